@@ -524,206 +524,454 @@ __device__ __noinline__ bool traverse(const DevScene &s, int32_t blasBase, V3 ra
 }
 
 // getBVHTraverseCode (intersect.wgsl.ts:213-629) as a restartable state
-// machine, for kernels that keep a queue of rays and give a lane a new ray as
-// soon as its current one has finished.  Each step() does exactly one of:
-// one node (a BLAS node of the current instance, or a TLAS node when no
-// instance is open: interior nodes of both levels run the same code, so lanes
-// at different levels stay together), or entering the next instance of the
-// current TLAS leaf.  Visit order, box tests, the `>` tie rule and the
-// self-hit and backface rules are those of traverse(), so the hits are
-// bit-identical to it.
+// machine, for warps that keep a queue of rays and give a lane a new ray as
+// soon as its current one has finished.  A lane's next piece of work is a
+// node to visit (interior, either level), an instance of the open TLAS leaf
+// to enter, or the triangles of a BLAS leaf; advance() runs one of these at a
+// time for all lanes of the warp that are at it.  A lane that waits only
+// waits: each ray's visit order, box tests, `>` tie rule and self-hit and
+// backface rules are those of traverse(), so the hits are bit-identical to it.
+//
+// What bounds it is issue slots at few active lanes.  With every lane taking
+// whatever step came next, an iteration ran the node code for ~20 lanes, the
+// instance code for ~6 and the triangle code for ~2, and the last two cost as
+// much as the first: 1,070 warp instructions a ray at 8.8 active lanes on the
+// instanced scene (1.45M bounce rays, 2.56 ms).  Repeating node visits while
+// enough lanes need one, the header word kept with each stack entry, paired
+// f32 box tests, and the shear of the watertight test computed at leaves
+// (2.3 a ray) instead of instances entered (11.4): 717 at 15 lanes, 1.9 ms.
+// Paired box tests alone are 6 % of the 1080p instanced render.
+//
+// Dense and sparse queues want different waits.  A warp with many rays behind
+// it goes back to the lanes at instances and leaves once fewer than
+// kNodeLanes are at nodes (12: 124 ms, 1: 130 ms for 8 samples of the 1080p
+// instanced scene); with few rays a warp's own latency is what counts, and it
+// finishes the node visits first (1: 31.3 ms, 12: 33.2 ms for the glass scene
+// at 1280x720, 6.4 against 6.9 for a 333x217 image).  Making lanes at leaves
+// and instances wait for company lost in both (8 and 4 lanes: 37 and 9 ms).
+constexpr uint32_t kNodeLanes = 12;
+constexpr uint32_t kDenseRays = 128;  // rays per warp from which kNodeLanes holds (64: the same within noise)
 constexpr int kTraversalStackEntries = 2 * MTC_MAX_STACK;
+
+// What a finished closest-hit query stores; the geometric normal is
+// recomputed from the triangle by whoever needs it (hitNormal).
+struct alignas(16) StoredHit {
+  float tMax, bary[3];
+  int32_t triangleIndex, insIdx, _pad[2];
+};
+
+// The candidate normal of the triangle test (intersect.wgsl.ts:1482-1493) for
+// the accepted triangle of a hit.
+MTD V3 hitNormal(const DevScene &s, int32_t triangleIndex, int32_t insIdx) {
+  const int32_t vertexOffset = asi(ld4(s.ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE).y);
+  const float4 r = ld4(s.bvh + triangleIndex);
+  const V3 p0 = vertexPosition(s, asi(r.x) + vertexOffset), p1 = vertexPosition(s, asi(r.y) + vertexOffset),
+           p2 = vertexPosition(s, asi(r.z) + vertexOffset);
+  return xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0)));
+}
+
+// The values of getShear(d, maxDim), the axes selected before the divisions
+// so that lanes of different dominant axes divide together.
+MTD V3 selectShear(V3 d, int maxDim) {
+  const float z = maxDim == 0 ? d.x : maxDim == 1 ? d.y : d.z;
+  const float x = maxDim == 0 ? d.y : maxDim == 1 ? d.z : d.x;
+  const float y = maxDim == 0 ? d.z : maxDim == 1 ? d.x : d.y;
+  return {xd(-x, z), xd(-y, z), __frcp_rn(z)};
+}
+
+// A query as its source hands it to a warp.
+struct RayQuery {
+  V3 o, d;
+  float limit;             // tMax at the start
+  int32_t tri, ins;        // the triangle a bounce leaves from (tri -1: none)
+  uint32_t payload, scene; // the source's own number of the query; its scene
+  bool doubleSided;
+};
+
+// Shared memory of one warp: a batch of queries fetched together (word k of
+// entry e at pending[k][e]) and the world-space ray of each lane's query, off
+// the registers that the node visits need.
+struct WarpRays {
+  float pending[14][32];
+  float ray[9][32];
+};
+
+// Three-operand minimum and maximum, and packed pairs of f32 operations, of
+// sm_100: each half rounds like the scalar instruction.
+MTD float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+MTD float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+MTD uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+MTD void unpack2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+MTD uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+MTD uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// A ray prepared for box tests: -origin and 1 / direction.
+struct BoxRay {
+  uint64_t oxy, ixy;
+  float oz, iz;
+  MTD void set(V3 o, V3 inv) {
+    oxy = pack2(-o.x, -o.y);
+    oz = -o.z;
+    ixy = pack2(inv.x, inv.y);
+    iz = inv.z;
+  }
+  MTD V3 origin() const {
+    V3 o;
+    unpack2(oxy, o.x, o.y);
+    return {-o.x, -o.y, -oz};
+  }
+};
+
+// intersectBox with its result split up: the entry and exit distances of the
+// slabs.  A box is hit when t0 <= min(t1, tMax) and t1 > 0; intersectBox then
+// returns t0 if positive, else t1.  (A min or max of all three axes is NaN
+// only when every axis is, for t0 and t1 alike: a miss in both forms.)
+MTD void boxSlabs(const BoxRay &r, ulonglong2 lo, ulonglong2 hi, float &t0, float &t1) {
+  float bx, by, bz, cx, cy, cz, ignored;
+  unpack2(mul2(add2(lo.x, r.oxy), r.ixy), bx, by);
+  unpack2(mul2(add2(hi.x, r.oxy), r.ixy), cx, cy);
+  unpack2(lo.y, bz, ignored);
+  unpack2(hi.y, cz, ignored);
+  bz = xm(xa(bz, r.oz), r.iz);
+  cz = xm(xa(cz, r.oz), r.iz);
+  t0 = max3(fminf(bx, cx), fminf(by, cy), fminf(bz, cz));
+  t1 = min3(fmaxf(bx, cx), fmaxf(by, cy), fmaxf(bz, cz));
+}
+MTD ulonglong2 ldNode(const float4 *p) { return __ldg(reinterpret_cast<const ulonglong2 *>(p)); }
+MTD int32_t nodeWord(ulonglong2 v) { return int32_t(uint32_t(v.y >> 32)); }
 
 template <bool shadow, bool kGpuLayout, bool kAlpha = false>
 struct RayTraversal {
-  const float4 *bvh, *ins, *mats;
-  const uint32_t *attr;
-  uint32_t vstride;
+  const DevScene *scene;
+  const float4 *bvh;
   int32_t blasBase;
-  V3 rayO, rayD, invD;
-  int bounces;
-  bool doubleSided;
+  float *world;  // rayO, rayD, 1 / rayD: word k at world[32 * k]
+  // The ray of the level being visited (world, or the open instance's), the
+  // instance-space direction, and what child pointers are relative to.
+  BoxRay ray;
+  V3 d;
+  int32_t rel;
   int32_t currentTri, currentIns;
-  // TLAS entries at [0, MTC_MAX_STACK), the current instance's BLAS entries
-  // at [MTC_MAX_STACK, 2 * MTC_MAX_STACK): two stacks of the reference's
-  // depth, addressed through one array of kTraversalStackEntries so TLAS and
-  // BLAS node visits share one code path.  The array belongs to the caller
-  // (a local array of the kernel): a dynamically indexed array inside this
-  // object would keep the whole object, ray and hit included, in local
-  // memory.
-  int32_t *stack;
-  int tlasTop, blasTop;
-  int32_t leafNode, io;
-  V3 o, d, linvD, shear;
-  int maxDim;
-  int32_t blasOffset, vertexOffset, sideMaterial, insIdx;
-  uint32_t blasLayout;
-  bool found;
-  TraversalHit h;
-  // Shadow queries of scenes with alpha: the scene and the path's sampler
-  // for alphaPasses, and the query's tMax to restore after a hit that does
-  // not occlude.  Null otherwise.
-  const DevScene *alphaScene;
+  bool doubleSided;
+  // Node entries (index, header word) of the TLAS, those of the open instance
+  // above them from `floor` on.  The array belongs to the caller (a local
+  // array of the kernel): a dynamically indexed array inside this object
+  // would keep the whole object, ray and hit included, in local memory.  Each
+  // level is bounded by the reference's stack depth.
+  int2 *stack;
+  int top, floor;
+  // What is worked on next: the node `cur` with its header word `ptr`.  An
+  // interior node has ptr >= 0; else the state tells a TLAS leaf (-ptr
+  // entries, or kEntriesLeft plus those an instance left to enter) from a
+  // BLAS leaf.
+  static constexpr int32_t kEntriesLeft = -(1 << 30);
+  int32_t cur, ptr;
+  enum : uint32_t { kTlas, kBlas, kDone, kIdle } state;
+  int32_t leafNode, io;   // open TLAS leaf and its last entry still to enter
+  int32_t vertexOffset, insIdx;
+  bool gpuNodes;          // the open instance's BLAS is BVH_GPU
+  float tMax;
+  V3 bary;
+  int32_t hitTri, hitIns;
+  // Shadow queries of scenes with alpha: the path's sampler for alphaPasses,
+  // and the query's tMax to restore after a hit that does not occlude.
   Sampler *alphaSmp;
   float tMaxInit;
 
-  MTD V3 position(int32_t i) const {
-    const uint32_t *w = attr + size_t(i) * vstride;
-    if (vstride == 4) {
-      float4 q = __ldg(reinterpret_cast<const float4 *>(w));
-      return {q.x, q.y, q.z};
-    }
-    return {asf(__ldg(w)), asf(__ldg(w + 1)), asf(__ldg(w + 2))};
+  MTD bool found() const { return hitTri >= 0; }
+  MTD V3 word3(int k) const { return {world[32 * k], world[32 * (k + 1)], world[32 * (k + 2)]}; }
+  MTD bool atNode() const { return ptr >= 0; }
+  MTD bool atLeaf() const { return ptr < 0 && state == kBlas; }
+  MTD bool atInstances() const { return ptr < 0 && state == kTlas; }
+  MTD void finish(uint32_t s) {
+    state = decltype(state)(s);
+    ptr = -1;
   }
 
-  // Starts a query; returns false when the root box is missed (nothing to do).
-  MTD bool begin(const DevScene &s, int32_t base, V3 ro, V3 rd, int b, bool ds, int32_t ct, int32_t ci, float tMax) {
-    bvh = s.bvh; ins = s.ins; mats = s.mats; attr = s.attr; vstride = s.vstride; blasBase = base;
-    rayO = ro; rayD = rd; bounces = b; doubleSided = ds; currentTri = ct; currentIns = ci;
+  // Takes entry `e` of the warp's batch, whose ray passed the root box.
+  MTD void begin(WarpRays &rays, uint32_t e, uint32_t lane, const DevScene &s, int32_t base) {
+    scene = &s; bvh = s.bvh; blasBase = base;
+    world = &rays.ray[0][lane];
+    float w[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) world[32 * k] = w[k] = rays.pending[k][e];
+    ray.set({w[0], w[1], w[2]}, {w[6], w[7], w[8]});
+    tMax = rays.pending[9][e];
+    currentTri = __float_as_int(rays.pending[10][e]);
+    currentIns = __float_as_int(rays.pending[11][e]);
+    doubleSided = __float_as_uint(rays.pending[13][e]) >> 31;
     if (kAlpha) {
-      alphaScene = nullptr;
       alphaSmp = nullptr;
       tMaxInit = tMax;
     }
-    h.tMax = tMax;
-    h.triangleIndex = -1;
-    h.insIdx = -1;
-    h.hitBary = v3(0.0f);
-    h.hitNormal = v3(0.0f);
-    found = false;
-    tlasTop = -1;
-    blasTop = -1;
-    io = -1;
-    leafNode = 0;
-    insIdx = -1;
-    blasOffset = 0;
-    blasLayout = 0;
-    invD = traversalInverse(rd);
-    if (intersectBox(rayO, xyz(ld4(bvh)), xyz(ld4(bvh + 1)), invD, h.tMax) > 0.0f) {
-      tlasTop = 0;
-      stack[0] = 0;
-      return true;
-    }
-    return false;
+    bary = v3(0.0f);
+    hitTri = -1; hitIns = -1;
+    gpuNodes = false;
+    rel = 0; top = 0; floor = 0;
+    state = kTlas;
+    cur = 0;
+    ptr = asi(ld4(bvh).w);
   }
 
-  // One traversal step; returns true when the query has finished.
-  MTD bool step() {
-    const bool blas = blasTop >= 0;
-    if (!blas) {
-      if (io >= 0) return enterInstance();
-      if (tlasTop < 0) return true;
-    }
-    // Pop one node of the current level.
-    int top = blas ? blasTop : tlasTop;
-    const int stackBase = blas ? MTC_MAX_STACK : 0;
-    int32_t node = stack[stackBase + top];
-    top--;
-    const int32_t base = blas ? blasBase : 0;
-    // Decode the node: BVH2 (TLAS, BLAS layout 0) keeps each child's box in
-    // the child; BVH_GPU (BLAS layout 2, intersect.wgsl.ts:453-497) keeps both
-    // child boxes in the node itself.
-    bool interior;
-    int32_t left = 0, right = 0, primitiveCount = 0, primitiveOffset = 0;
-    float4 lmin, lmax, rmin, rmax;
-    if (kGpuLayout && blas && blasLayout == 2u) {
-      lmin = ld4(bvh + node + base);
-      lmax = ld4(bvh + node + base + 1);
-      rmin = ld4(bvh + node + base + 2);
-      rmax = ld4(bvh + node + base + 3);
-      int32_t count = int32_t(asu(rmin.w));
-      interior = count <= 0;
-      left = blasOffset + int32_t(asu(lmin.w) * 4u);
-      right = blasOffset + int32_t(asu(lmax.w) * 4u);
-      primitiveCount = count;
-      primitiveOffset = base + blasOffset + int32_t(asu(rmax.w));
+  // Takes the next node off the stack; at the end of an instance, what is
+  // left of its TLAS leaf (enter() goes on from there).
+  MTD void pop() {
+    if (top > floor) {
+      const int2 e = stack[--top];
+      cur = e.x;
+      ptr = e.y;
+    } else if (state == kBlas) {
+      state = kTlas;
+      cur = leafNode;
+      ptr = kEntriesLeft + io + 1;
     } else {
-      int32_t p = asi(ld4(bvh + node + base).w);
-      interior = p >= 0;
-      left = node + 2;
-      right = blas ? p + blasOffset : p;
-      primitiveCount = -p;
-      primitiveOffset = node + base + 2;
-      if (interior) {
-        lmin = ld4(bvh + left + base);
-        lmax = ld4(bvh + left + 1 + base);
-        rmin = ld4(bvh + right + base);
-        rmax = ld4(bvh + right + 1 + base);
-      }
+      finish(kDone);
     }
-    if (interior) {
-      // Interior node at either level (one code path for both).
-      visitInterior(bvh, base, blas ? blasOffset : 0, !(kGpuLayout && blas && blasLayout == 2u), blas ? o : rayO,
-                    blas ? linvD : invD, h.tMax, left, right, lmin, lmax, rmin, rmax, stack + stackBase, top);
-      if (blas) blasTop = top; else tlasTop = top;
-      return false;
-    }
-    if (blas) blasTop = top; else tlasTop = top;
-    if (!blas) {
-      leafNode = node;
-      io = primitiveCount - 1;
-      return false;
-    }
-    for (int32_t k = 0; k < primitiveCount; k++) {
-      int32_t triangleIndex = primitiveOffset + k;
-      if (bounces > 0 && triangleIndex == currentTri && insIdx == currentIns) continue;
-      float4 r3 = ld4(bvh + triangleIndex);
-      V3 p0 = position(asi(r3.x) + vertexOffset);
-      V3 p1 = position(asi(r3.y) + vertexOffset);
-      V3 p2 = position(asi(r3.z) + vertexOffset);
-      V3 bary;
-      float t = intersectTriangle(o, p0, p1, p2, maxDim, shear, h.tMax, bary);
-      if (!(t > 0.0f)) continue;
-      V3 candidateNormal = xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0)));
-      if (!doubleSided) {
-        bool matDoubleSided = __ldg(&mats[size_t(sideMaterial) * MTC_MATERIAL_VEC4_ROWS + 23].z) > 0.5f;
-        if (!matDoubleSided && xdot(candidateNormal, d) > 0.0f) continue;
-      }
-      h.hitNormal = candidateNormal;
-      h.tMax = t;
-      h.hitBary = bary;
-      if (shadow) {
-        if (kAlpha && alphaSmp &&
-            !alphaPasses(*alphaScene, sideMaterial, triangleIndex, asi(r3.x) + vertexOffset,
-                         asi(r3.y) + vertexOffset, asi(r3.z) + vertexOffset, bary, o + d * t, candidateNormal,
-                         *alphaSmp)) {
-          h.tMax = tMaxInit;
-          continue;
-        }
-        found = true;
-        return true;
-      }
-      h.triangleIndex = triangleIndex;
-      h.insIdx = insIdx;
-    }
-    return false;
   }
 
-  // Next instance entry of the current TLAS leaf (descending, as the WGSL's
-  // leaf loop): the ray in instance space and its watertight-test shear.
-  MTD bool enterInstance() {
-    float4 rec = ld4(bvh + leafNode + 2 + io);
+  // The interior visit at either level (intersect.wgsl.ts:265-300, :439-624):
+  // box-test both children and go on with the one the reference pushes last
+  // (the nearer, by the `>` rule), the other one on the stack.
+  MTD void visit() {
+    int32_t left = cur + 2, right = ptr + rel;
+    ulonglong2 lmin, lmax, rmin, rmax;
+    int32_t lptr, rptr;
+    if (kGpuLayout && gpuNodes) {
+      // BVH_GPU (BLAS layout 2, intersect.wgsl.ts:453-497): both child boxes
+      // in the node, which may itself be a leaf.
+      lmin = ldNode(bvh + cur);
+      lmax = ldNode(bvh + cur + 1);
+      rmin = ldNode(bvh + cur + 2);
+      rmax = ldNode(bvh + cur + 3);
+      const int32_t count = nodeWord(rmin);
+      if (count > 0) {
+        cur = rel + nodeWord(rmax) - 2;  // records at cur + 2
+        ptr = -count;
+        return;
+      }
+      left = rel + nodeWord(lmin) * 4;
+      right = rel + nodeWord(lmax) * 4;
+      lptr = rptr = 0;
+    } else {
+      lmin = ldNode(bvh + left);
+      lmax = ldNode(bvh + left + 1);
+      rmin = ldNode(bvh + right);
+      rmax = ldNode(bvh + right + 1);
+      lptr = nodeWord(lmin);
+      rptr = nodeWord(rmin);
+    }
+    float l0, l1, r0, r1;
+    boxSlabs(ray, lmin, lmax, l0, l1);
+    boxSlabs(ray, rmin, rmax, r0, r1);
+    const bool hitL = !(l0 > fminf(l1, tMax)) && l1 > 0.0f, hitR = !(r0 > fminf(r1, tMax)) && r1 > 0.0f;
+    // The farther child is pushed first; without room for a second entry it
+    // is the only one.
+    const bool both = hitL && hitR, leftFar = (l0 > 0.0f ? l0 : l1) > (r0 > 0.0f ? r0 : r1);
+    const bool push = both && top - floor + 1 < MTC_MAX_STACK;
+    const bool nextLeft = both ? leftFar != push : hitL;
+    if (push) stack[top++] = leftFar ? make_int2(left, lptr) : make_int2(right, rptr);
+    cur = nextLeft ? left : right;
+    ptr = nextLeft ? lptr : rptr;
+    if (!(hitL || hitR)) pop();
+  }
+
+  // Next instance entry of the open TLAS leaf (descending, as the WGSL's
+  // leaf loop): the ray in instance space, its BLAS root taken.  Without one,
+  // the next TLAS node.
+  MTD void enter() {
+    if (ptr < kEntriesLeft / 2) {  // an instance was finished
+      io = ptr - kEntriesLeft - 1;
+    } else {
+      leafNode = cur;
+      io = -ptr - 1;
+    }
+    if (io < 0) {
+      floor = 0;
+      rel = 0;
+      gpuNodes = false;
+      ray.set(word3(0), word3(6));
+      pop();
+      return;
+    }
+    const float4 rec = ld4(bvh + leafNode + 2 + io);
     io--;
     insIdx = asi(rec.x);
-    int32_t blasRoot = asi(rec.y);
-    const float4 *insv = ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE;
-    float4 insData = ld4(insv);
-    uint32_t encoded = asu(insData.x);
-    blasLayout = encoded >> 30;
-    if (blasLayout != 0u && !(kGpuLayout && blasLayout == 2u)) return false;  // TinyBVH bvh4 / cwbvh are not consumed
-    float4 c0 = ld4(insv + 1), c1 = ld4(insv + 2), c2 = ld4(insv + 3), c3 = ld4(insv + 4);
-    o = xmat4(c0, c1, c2, c3, rayO, 1.0f);
-    d = xmat4(c0, c1, c2, c3, rayD, 0.0f);
-    linvD = traversalInverse(d);
-    maxDim = maxDimension(vabs(d));
-    shear = getShear(d, maxDim);
-    blasOffset = int32_t(encoded & 0x3fffffffu);
+    const float4 *insv = scene->ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE;
+    const float4 insData = ld4(insv);
+    const float4 c0 = ld4(insv + 1), c1 = ld4(insv + 2), c2 = ld4(insv + 3), c3 = ld4(insv + 4);
+    cur = asi(rec.y) + blasBase;
+    const uint32_t encoded = asu(insData.x), layout = encoded >> 30;
+    floor = top;
+    if (layout != 0u && !(kGpuLayout && layout == 2u)) {  // TinyBVH bvh4 / cwbvh are not consumed
+      cur = leafNode;
+      ptr = kEntriesLeft + io + 1;
+      return;
+    }
+    gpuNodes = kGpuLayout && layout == 2u;
+    ptr = gpuNodes ? 0 : asi(ld4(bvh + cur).w);
+    d = xmat4(c0, c1, c2, c3, word3(3), 0.0f);
+    ray.set(xmat4(c0, c1, c2, c3, word3(0), 1.0f), traversalInverse(d));
+    rel = blasBase + int32_t(encoded & 0x3fffffffu);
     vertexOffset = asi(insData.y);
-    sideMaterial = asi(insData.z) >> 8;
-    blasTop = 0;
-    stack[MTC_MAX_STACK] = blasRoot;
-    return false;
+    state = kBlas;
+  }
+
+  // The triangles of a BLAS leaf.
+  MTD void leaf() {
+    const int maxDim = maxDimension(vabs(d));
+    const V3 shear = selectShear(d, maxDim), o = ray.origin();
+    const int32_t last = cur + 2 - ptr;
+    for (int32_t triangleIndex = cur + 2; triangleIndex < last; triangleIndex++) {
+      if (triangleIndex == currentTri && insIdx == currentIns) continue;
+      const float4 r = ld4(bvh + triangleIndex);
+      const int32_t i0 = asi(r.x) + vertexOffset, i1 = asi(r.y) + vertexOffset, i2 = asi(r.z) + vertexOffset;
+      const V3 p0 = vertexPosition(*scene, i0), p1 = vertexPosition(*scene, i1), p2 = vertexPosition(*scene, i2);
+      V3 b;
+      const float t = intersectTriangle(o, p0, p1, p2, maxDim, shear, tMax, b);
+      if (!(t > 0.0f)) continue;
+      if (!shadow && !doubleSided) {
+        const int32_t material = asi(ld4(scene->ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE).z) >> 8;
+        const bool both = __ldg(&scene->mats[size_t(material) * MTC_MATERIAL_VEC4_ROWS + 23].z) > 0.5f;
+        if (!both && xdot(xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0))), d) > 0.0f) continue;
+      }
+      tMax = t;
+      if (shadow) {
+        if (kAlpha && alphaSmp) {
+          const int32_t material = asi(ld4(scene->ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE).z) >> 8;
+          if (!alphaPasses(*scene, material, triangleIndex, i0, i1, i2, b, o + d * t,
+                           xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0))), *alphaSmp)) {
+            tMax = tMaxInit;
+            continue;
+          }
+        }
+        hitTri = triangleIndex;
+        finish(kDone);
+        return;
+      }
+      bary = b;
+      hitTri = triangleIndex;
+      hitIns = insIdx;
+    }
+    pop();
+  }
+
+  // One round of the warp's busy lanes (all 32 lanes call it): leaves, then
+  // instances, then at least one node visit and up to `steps` while
+  // `nodeLanes` lanes need one.
+  MTD void advance(uint32_t steps, uint32_t nodeLanes) {
+    if (__any_sync(0xffffffffu, atLeaf())) {
+      if (atLeaf()) leaf();
+      __syncwarp();
+    }
+    if (__any_sync(0xffffffffu, atInstances())) {
+      if (atInstances()) enter();
+      __syncwarp();
+    }
+    unsigned node = __ballot_sync(0xffffffffu, atNode());
+    for (uint32_t k = 0; node && k < steps; k++) {
+      if (atNode()) visit();
+      __syncwarp();
+      node = __ballot_sync(0xffffffffu, atNode());
+      if (uint32_t(__popc(node)) < nodeLanes) break;
+    }
   }
 };
+
+// Drains queries [0, count) of a source with the calling warp (all 32 lanes
+// call it).  The warp takes up to 32 queries at a time off the shared counter
+// `next`, every lane reading one of them, so that the chain of dependent
+// loads behind a query (counter, queue, record, scene) is paid once a batch
+// instead of by a whole warp at each lane's refill.  Where there are fewer
+// queries than lanes, the batches shrink so that every warp gets some.
+//
+// The source has scene(i) and blasBase(i), read(t, query): false when query t
+// is answered without a traversal, missed(query), and done(traversal,
+// payload) for a finished one, and alpha(traversal, payload, scene).
+template <bool shadow, bool kGpuLayout, bool kAlpha, class Source>
+MTD void traceQueue(Source &src, uint32_t count, uint32_t *next, uint32_t refillLanes, uint32_t steps,
+                    WarpRays &rays) {
+  int2 stack[kTraversalStackEntries];
+  RayTraversal<shadow, kGpuLayout, kAlpha> rt;
+  rt.stack = stack;
+  rt.finish(rt.kIdle);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+  const uint32_t batch = min(32u, max(1u, (count + warps - 1u) / warps));
+  const uint32_t nodeLanes = count / warps >= kDenseRays ? kNodeLanes : 1u;
+  uint32_t payload = 0, head = 0, have = 0;
+  bool exhausted = false;
+  for (;;) {
+    const unsigned idle = __ballot_sync(0xffffffffu, rt.state == rt.kIdle);
+    if (idle == 0xffffffffu && exhausted && head == have) break;
+    // Refill once enough lanes wait (or none is left tracing).
+    if (uint32_t(__popc(idle)) >= refillLanes || idle == 0xffffffffu) {
+      if (head == have && !exhausted) {
+        uint32_t first = 0;
+        if (lane == 0) first = atomicAdd(next, batch);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        exhausted = first >= count || count - first <= batch;
+        RayQuery q;
+        bool keep = lane < batch && first < count && lane < count - first && src.read(first + lane, q);
+        V3 inv = v3(0.0f);
+        if (keep) {
+          const float4 *bvh = src.scene(q.scene).bvh;
+          inv = traversalInverse(q.d);
+          if (!(intersectBox(q.o, xyz(ld4(bvh)), xyz(ld4(bvh + 1)), inv, q.limit) > 0.0f)) {
+            src.missed(q);
+            keep = false;
+          }
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const uint32_t e = __popc(kept & ((1u << lane) - 1u));
+          const float w[14] = {q.o.x, q.o.y, q.o.z, q.d.x, q.d.y, q.d.z, inv.x, inv.y, inv.z, q.limit,
+                               __int_as_float(q.tri), __int_as_float(q.ins), __uint_as_float(q.payload),
+                               __uint_as_float(q.scene | (q.doubleSided ? 0x80000000u : 0u))};
+#pragma unroll
+          for (int k = 0; k < 14; k++) rays.pending[k][e] = w[k];
+        }
+        __syncwarp();
+        head = 0;
+        have = __popc(kept);
+      }
+      const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+      if (rt.state == rt.kIdle && head + rank < have) {
+        const uint32_t e = head + rank;
+        payload = __float_as_uint(rays.pending[12][e]);
+        const uint32_t i = __float_as_uint(rays.pending[13][e]) & 0x7fffffffu;
+        rt.begin(rays, e, lane, src.scene(i), src.blasBase(i));
+        if (kAlpha) src.alpha(rt, payload, i);
+      }
+      __syncwarp();
+      head = min(have, head + uint32_t(__popc(idle)));
+    }
+    rt.advance(steps, nodeLanes);
+    if (rt.state == rt.kDone) {
+      src.done(rt, payload);
+      rt.finish(rt.kIdle);
+    }
+    __syncwarp();
+  }
+}
 
 }  // namespace mt

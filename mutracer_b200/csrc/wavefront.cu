@@ -76,7 +76,7 @@ struct StreamView {
   StreamQueues *q;
   Slot *slots;
   SpectralState *spectral;  // per slot, used by spectral jobs only
-  TraversalHit *hits;
+  StoredHit *hits;
   uint32_t *rayQueue[2];
   uint32_t *shadowQueue, *finishQueue;
   uint32_t *keys, *sortedQueue;   // material-class key per slot; extension queue ordered by key
@@ -160,9 +160,9 @@ __device__ __forceinline__ BsdfContext bsdfContext(const JobData &J) {
 // MaterialBuffer rows that getMaterial reads (materialLayoutSchema.ts:23-150).
 constexpr uint32_t kClasses = 64;
 
-__device__ __forceinline__ uint32_t materialClass(const JobData &J, const TraversalHit &h) {
-  if (h.insIdx < 0) return 0u;
-  const float4 *insv = J.s.ins + size_t(h.insIdx) * MTC_INSTANCE_VEC4_STRIDE;
+__device__ __forceinline__ uint32_t materialClass(const JobData &J, int32_t insIdx) {
+  if (insIdx < 0) return 0u;
+  const float4 *insv = J.s.ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE;
   int32_t mi = asi(ld4(insv).z) >> 8;
   if (uint32_t(mi) >= J.s.matCount) mi = 0;
   const float4 *d = J.s.mats + size_t(mi) * MTC_MATERIAL_VEC4_ROWS;
@@ -245,6 +245,11 @@ __device__ bool claimPixel(const StreamView &v, uint32_t s) {
   return false;
 }
 
+// Adds the NEE contribution of a slot whose shadow query was not occluded.
+__device__ __forceinline__ void addUnoccluded(PathSample &ps, const ShadowQuery &q) {
+  if (q.valid) ps.path.li += q.contribution;
+}
+
 __global__ void __launch_bounds__(kStreamThreads) k_wf_seed(StreamView v, uint32_t regroup0) {
   if (blockIdx.x == 0 && threadIdx.x == 0) v.q->regroup = regroup0;
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < v.slotCount; s += gridDim.x * blockDim.x) {
@@ -257,18 +262,62 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_seed(StreamView v, uint32
 // has finished takes the next queued ray at once, so a warp is not held by
 // its slowest ray (traversal lengths differ by an order of magnitude here).
 // Resident CTAs per SM of the traversal kernels: the closest-hit kernel at
-// 5 holds its traversal state in 95 registers without spilling, the shadow
-// kernel at 6 in 80 (measured 2 % and 0.8 % faster than 8 CTAs at 64
-// registers with spills; 4 is 3.5 % slower).
+// 5 holds its traversal state in 87 registers and the shadow kernel at 6 in
+// 78, without spilling (6 and 7 CTAs: within 1 % on the 1080p instanced
+// scene, 4 % slower on the glass scene).
 #ifndef MT_EXTEND_MIN_BLOCKS
 #define MT_EXTEND_MIN_BLOCKS 5
 #endif
 #ifndef MT_SHADOW_MIN_BLOCKS
 #define MT_SHADOW_MIN_BLOCKS 6
 #endif
+// The extension rays of one event iteration.
+struct ExtendSource {
+  const StreamView &v;
+  const uint32_t *queue;
+  uint32_t rays;
+  MTD const DevScene &scene(uint32_t job) const { return v.jobs[job].s; }
+  MTD int32_t blasBase(uint32_t job) const { return v.jobs[job].u.blas_offset; }
+  MTD void store(uint32_t s, float t, V3 bary, int32_t tri, int32_t ins) const {
+    float4 *hit = reinterpret_cast<float4 *>(v.hits + s);
+    hit[0] = make_float4(t, bary.x, bary.y, bary.z);
+    hit[1] = make_float4(__int_as_float(tri), __int_as_float(ins), 0.0f, 0.0f);
+  }
+  MTD bool read(uint32_t t, RayQuery &q) {
+    const uint32_t s = queue[t];
+    if (s >= v.slotCount) return false;  // not reachable with consistent queue counts
+    const Slot &sl = v.slots[s];
+    const JobData &J = v.jobs[sl.job];
+    q.payload = s;
+    q.scene = sl.job;
+    // traceExtension: an empty scene is a miss without a traversal, and a
+    // spectral wavelength path restarting at the shared primary vertex
+    // traces nothing.
+    if (J.u.is_empty > 0 || (isSpectral(J) && reusesPrimary(J, sl.ps, v.spectral[s].primaryReady)) ||
+        (alphaSplit(J) && v.spectral[s].frontPending)) {
+      missed(q);
+      return false;
+    }
+    rays++;
+    q.o = sl.ps.path.ray.o;
+    q.d = sl.ps.path.ray.d;
+    q.limit = RAY_MAX_DISTANCE;
+    q.tri = sl.ps.depth > 0 ? sl.ps.si.triangleIndex : -1;
+    q.ins = sl.ps.si.instanceIndex;
+    q.doubleSided = sl.ps.event != 0;
+    return true;
+  }
+  MTD void missed(const RayQuery &q) const { store(q.payload, RAY_MAX_DISTANCE, v3(0.0f), -1, -1); }
+  template <class T>
+  MTD void done(const T &rt, uint32_t s) const { store(s, rt.tMax, rt.bary, rt.hitTri, rt.hitIns); }
+  template <class T>
+  MTD void alpha(T &, uint32_t, uint32_t) const {}
+};
+
 template <bool kGpuLayout>
 __global__ void __launch_bounds__(kStreamThreads, MT_EXTEND_MIN_BLOCKS)
     k_wf_extend(StreamView v) {
+  __shared__ WarpRays rays[kStreamThreads / 32];
   const uint32_t cur = v.q->cur;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     v.q->rayCount[cur ^ 1u] = 0;
@@ -276,7 +325,6 @@ __global__ void __launch_bounds__(kStreamThreads, MT_EXTEND_MIN_BLOCKS)
     v.q->finishCount = 0;
   }
   const uint32_t n = v.q->rayCount[cur];
-  const uint32_t *queue = v.sortRays ? v.sortedRays : v.rayQueue[cur];
   if (v.sortRays && blockIdx.x == 0) {
     // The ray-key counts of this queue were consumed by k_wf_sort_rays.
     for (uint32_t k = threadIdx.x; k < kRayKeys; k += blockDim.x) {
@@ -284,57 +332,10 @@ __global__ void __launch_bounds__(kStreamThreads, MT_EXTEND_MIN_BLOCKS)
       v.rayKeyCursor[k] = 0;
     }
   }
-  int32_t stack[kTraversalStackEntries];
-  RayTraversal<false, kGpuLayout> rt;
-  rt.stack = stack;
-  uint32_t s = 0, ext = 0;
-  bool busy = false, exhausted = false;
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !busy && !exhausted);
-    const unsigned live = __ballot_sync(0xffffffffu, busy);
-    if (!idle && !live) break;
-    // Refill once enough lanes wait (or none is left tracing).
-    if (idle && (uint32_t(__popc(idle)) >= v.refillLanes || !live)) {
-      if (busy || exhausted) continue;
-      uint32_t t = takeUnit(&v.q->extendNext);
-      if (t >= n) {
-        exhausted = true;
-      } else if ((s = queue[t]) >= v.slotCount) {
-        // Not reachable with consistent queue counts; never index past the slots.
-      } else {
-        const Slot &sl = v.slots[s];
-        const JobData &J = v.jobs[sl.job];
-        // traceExtension: an empty scene is a miss without a traversal, and a
-        // spectral wavelength path restarting at the shared primary vertex
-        // traces nothing.
-        if (J.u.is_empty > 0 || (isSpectral(J) && reusesPrimary(J, sl.ps, v.spectral[s].primaryReady)) ||
-            (alphaSplit(J) && v.spectral[s].frontPending)) {
-          TraversalHit none;
-          none.tMax = RAY_MAX_DISTANCE;
-          none.triangleIndex = -1;
-          none.insIdx = -1;
-          v.hits[s] = none;
-        } else {
-          ext++;
-          if (rt.begin(J.s, J.u.blas_offset, sl.ps.path.ray.o, sl.ps.path.ray.d, sl.ps.depth, sl.ps.event != 0,
-                       sl.ps.si.triangleIndex, sl.ps.si.instanceIndex, RAY_MAX_DISTANCE)) {
-            busy = true;
-          } else {
-            v.hits[s] = rt.h;
-          }
-        }
-      }
-      continue;
-    }
-    // Several steps between refill checks: the votes cost as much as a node.
-    bool finished = false;
-    for (uint32_t k = 0; k < v.stepsPerCheck && busy && !finished; k++) finished = rt.step();
-    if (finished) {
-      v.hits[s] = rt.h;
-      busy = false;
-    }
-  }
-  flush(v, ext, 0, 0);
+  ExtendSource src{v, v.sortRays ? v.sortedRays : v.rayQueue[cur], 0u};
+  traceQueue<false, kGpuLayout, false>(src, n, &v.q->extendNext, v.refillLanes, v.stepsPerCheck,
+                                       rays[threadIdx.x / 32u]);
+  flush(v, src.rays, 0, 0);
 }
 
 // Material class of every traced ray of this iteration (read from its hit),
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_classify(StreamView v) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const uint32_t s = queue[t];
     if (s >= v.slotCount) continue;
-    countClass(v, s, materialClass(v.jobs[v.slots[s].job], v.hits[s]));
+    countClass(v, s, materialClass(v.jobs[v.slots[s].job], v.hits[s].insIdx));
   }
 }
 
@@ -441,7 +442,15 @@ __global__ void __launch_bounds__(kStreamThreads, MT_SHADE_MIN_BLOCKS)
     c.shadow.valid = false;
     alignas(16) PathSample ps;
     copyPathSample(ps, sl.ps);
-    TraversalHit h = v.hits[s];
+    addUnoccluded(ps, sl.shadow);
+    const float4 h0 = __ldcg(reinterpret_cast<const float4 *>(v.hits + s));
+    const float4 h1 = __ldcg(reinterpret_cast<const float4 *>(v.hits + s) + 1);
+    TraversalHit h;
+    h.tMax = h0.x;
+    h.hitBary = {h0.y, h0.z, h0.w};
+    h.triangleIndex = asi(h1.x);
+    h.insIdx = asi(h1.y);
+    h.hitNormal = h.insIdx >= 0 ? hitNormal(J.s, h.triangleIndex, h.insIdx) : v3(0.0f);
     bool ended = isSpectral(J)   ? shadeStepSpectral(c, ps, v.spectral[s], h)
                  : alphaSplit(J) ? shadeStepAlpha(c, ps, v.spectral[s], h)
                                  : shadeStep(c, ps, v.spectral[s], h);
@@ -455,69 +464,49 @@ __global__ void __launch_bounds__(kStreamThreads, MT_SHADE_MIN_BLOCKS)
   flush(v, 0, 0, 0);
 }
 
-// NEE visibility of the queued shadow rays (intersectSceneShadow and
-// resolveShadow), persistent like k_wf_extend.
+// NEE visibility of the queued shadow rays (intersectSceneShadow).  An
+// occluded query is marked in its slot, a store that nothing waits for; the
+// kernel that reads the slot next adds the contributions of the others
+// (addUnoccluded, the sum of resolveShadow).
+struct ShadowSource {
+  const StreamView &v;
+  uint32_t rays;
+  MTD const DevScene &scene(uint32_t job) const { return v.jobs[job].s; }
+  MTD int32_t blasBase(uint32_t job) const { return v.jobs[job].u.blas_offset; }
+  MTD bool read(uint32_t t, RayQuery &q) {
+    const uint32_t s = v.shadowQueue[t];
+    const Slot &sl = v.slots[s];
+    q.payload = s;
+    q.scene = sl.job;
+    if (v.jobs[sl.job].u.is_empty > 0) return false;
+    rays++;
+    q.o = sl.shadow.ray.o;
+    q.d = sl.shadow.ray.d;
+    q.limit = fminf(fmaxf(sl.shadow.maxDistance, 0.0f), RAY_MAX_DISTANCE);
+    q.tri = sl.shadow.triangleIndex;
+    q.ins = sl.shadow.instanceIndex;
+    q.doubleSided = true;
+    return true;
+  }
+  MTD void missed(const RayQuery &) const {}
+  template <class T>
+  MTD void done(const T &rt, uint32_t s) const {
+    if (rt.found()) v.slots[s].shadow.valid = false;
+  }
+  // Coverage draws advance the path's own sampler, in place.
+  template <class T>
+  MTD void alpha(T &rt, uint32_t s, uint32_t job) const {
+    if (v.jobs[job].s.flags & MTC_SCENE_HAS_ALPHA) rt.alphaSmp = &v.slots[s].smp;
+  }
+};
+
 template <bool kGpuLayout, bool kAlpha>
 __global__ void __launch_bounds__(kStreamThreads, MT_SHADOW_MIN_BLOCKS) k_wf_shadow(StreamView v) {
-  const uint32_t n = v.q->shadowCount;
-  int32_t stack[kTraversalStackEntries];
-  RayTraversal<true, kGpuLayout, kAlpha> rt;
-  rt.stack = stack;
-  uint32_t s = 0, shadowRays = 0;
-  bool busy = false, exhausted = false;
-  for (;;) {
-    bool done = false;
-    const unsigned idle = __ballot_sync(0xffffffffu, !busy && !exhausted);
-    const unsigned live = __ballot_sync(0xffffffffu, busy);
-    if (!idle && !live) break;
-    const bool refill = idle && (uint32_t(__popc(idle)) >= v.refillLanes || !live);
-    if (refill && !busy && !exhausted) {
-      uint32_t t = takeUnit(&v.q->shadowNext);
-      if (t >= n) {
-        exhausted = true;
-      } else {
-        s = v.shadowQueue[t];
-        const Slot &sl = v.slots[s];
-        const JobData &J = v.jobs[sl.job];
-        const ShadowQuery &q = sl.shadow;
-        if (J.u.is_empty > 0) {
-          rt.found = false;
-          done = true;
-        } else {
-          shadowRays++;
-          float tMax = fminf(fmaxf(q.maxDistance, 0.0f), RAY_MAX_DISTANCE);
-          if (rt.begin(J.s, J.u.blas_offset, q.ray.o, q.ray.d, 1, true, q.triangleIndex, q.instanceIndex, tMax)) {
-            busy = true;
-            // Coverage draws advance the path's own sampler, in place.
-            if (kAlpha && (J.s.flags & MTC_SCENE_HAS_ALPHA)) {
-              rt.alphaScene = &J.s;
-              rt.alphaSmp = &v.slots[s].smp;
-            }
-          } else {
-            done = true;
-          }
-        }
-      }
-    }
-    if (!refill && busy) {
-      bool finished = false;
-      for (uint32_t k = 0; k < v.stepsPerCheck && !finished; k++) finished = rt.step();
-      if (finished) {
-        busy = false;
-        done = true;
-      }
-    }
-    if (done) {
-      Slot &sl = v.slots[s];
-      if (!rt.found) {
-        V3 li = sl.ps.path.li;
-        li += sl.shadow.contribution;
-        sl.ps.path.li = li;
-      }
-      sl.shadow.valid = false;
-    }
-  }
-  flush(v, 0, shadowRays, 0);
+  __shared__ WarpRays rays[kStreamThreads / 32];
+  ShadowSource src{v, 0u};
+  traceQueue<true, kGpuLayout, kAlpha>(src, v.q->shadowCount, &v.q->shadowNext, v.refillLanes, v.stepsPerCheck,
+                                       rays[threadIdx.x / 32u]);
+  flush(v, 0, src.rays, 0);
 }
 
 __global__ void __launch_bounds__(kStreamThreads) k_wf_finish(StreamView v) {
@@ -532,19 +521,25 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_finish(StreamView v) {
     alignas(16) PathSample ps;
     if (isSpectral(J) || alphaSplit(J)) {
       copyPathSample(ps, sl.ps);
+      addUnoccluded(ps, sl.shadow);
       if ((isSpectral(J) && !finishWavelength(J, ps, v.spectral[s])) ||
           (alphaSplit(J) && !finishAlphaSplit(J, ps, v.spectral[s]))) {
         // The next wavelength path, or the front path, of this sample starts
         // at event 0.
         copyPathSample(sl.ps, ps);
+        sl.shadow.valid = false;
         enqueueRay(v, cur ^ 1u, s);
         continue;
       }
       endSample(J, sl.x + sl.y * J.width, ps);
     } else {
-      // The accumulation reads a dozen words of the path sample: from the
-      // slot itself rather than a copy of all of it.
-      endSample(J, sl.x + sl.y * J.width, sl.ps);
+      // The accumulation reads a dozen words of the path sample: only these
+      // are copied.
+      ps.path.li = sl.ps.path.li;
+      ps.path.alpha = sl.ps.path.alpha;
+      ps.aux = sl.ps.aux;
+      addUnoccluded(ps, sl.shadow);
+      endSample(J, sl.x + sl.y * J.width, ps);
     }
     paths++;
     bool again;
@@ -554,6 +549,7 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_finish(StreamView v) {
       beginSample(c, sl.x, sl.y, ps, v.spectral[s]);
       copyPathSample(sl.ps, ps);
       sl.smp = c.smp;
+      sl.shadow.valid = false;
       again = true;
     } else {
       again = claimPixel(v, s);
@@ -602,7 +598,7 @@ StreamLayout layout(uint32_t capacity, uint32_t slots) {
   L.spectral = off;
   off += roundUp(size_t(slots) * sizeof(SpectralState));
   L.hits = off;
-  off += roundUp(size_t(slots) * sizeof(TraversalHit));
+  off += roundUp(size_t(slots) * sizeof(StoredHit));
   L.rayQueues = off;
   off += 2 * roundUp(size_t(slots) * 4);
   L.shadowQueue = off;
@@ -918,7 +914,7 @@ mt_status streamLaunch(const void *table, uint32_t capacity, const mtc_stream_co
   v.q = reinterpret_cast<StreamQueues *>(base + L.queues);
   v.slots = reinterpret_cast<Slot *>(base + L.slots);
   v.spectral = reinterpret_cast<SpectralState *>(base + L.spectral);
-  v.hits = reinterpret_cast<TraversalHit *>(base + L.hits);
+  v.hits = reinterpret_cast<StoredHit *>(base + L.hits);
   v.rayQueue[0] = reinterpret_cast<uint32_t *>(base + L.rayQueues);
   v.rayQueue[1] = reinterpret_cast<uint32_t *>(base + L.rayQueues + roundUp(size_t(shape.slots) * 4));
   v.shadowQueue = reinterpret_cast<uint32_t *>(base + L.shadowQueue);
