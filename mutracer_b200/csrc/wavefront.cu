@@ -60,7 +60,8 @@ struct StreamQueues {
   uint32_t iterations;
   uint32_t limitHit;
   uint32_t more;
-  uint32_t _pad[52];
+  uint32_t shadeNext;        // next chunk of the shading queue to hand to a block
+  uint32_t _pad[51];
 };
 static_assert(sizeof(StreamQueues) == 256, "queue header size");
 
@@ -383,6 +384,12 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_sort_rays(StreamView v) {
   }
 }
 
+// A long shading queue starts with the costly classes, so that misses and
+// plain diffuse hits are left for its tail (119.5 against 124.3 ms, 8 samples
+// of the 1080p instanced scene, 2M rays); one of a few chunks a block keeps
+// the ascending order (30.9 against 32.4 ms, Cornell box, 262k rays).
+constexpr uint32_t kCostlyFirstRays = 1u << 19;
+
 // Orders the extension queue by material class (counting sort on the keys
 // counted by k_wf_extend), so that the warps shading at any one time run the
 // same BSDF code.  The order of slots inside a class is arbitrary; it cannot
@@ -392,9 +399,11 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_regroup(StreamView v) {
   countLaunch(v);
   if (!v.q->regroup) return;
   const uint32_t cur = v.q->cur;
+  const bool costlyFirst = v.q->rayCount[cur] >= kCostlyFirstRays;
   if (threadIdx.x == 0) {
     uint32_t acc = 0;
-    for (uint32_t k = 0; k < kClasses; k++) {
+    for (uint32_t i = 0; i < kClasses; i++) {
+      const uint32_t k = costlyFirst ? kClasses - 1u - i : i;
       offset[k] = acc;
       acc += v.classCount[k];
     }
@@ -414,13 +423,22 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_regroup(StreamView v) {
   }
 }
 
-// Shading at 8 CTAs per SM (64 registers, 32 warps): more spilled state, but
-// twice the warps to hide its latency (measured: 4 CTAs at 128 registers
-// 6 % slower on the headline, 10-16 CTAs 2-4 % slower).
+// Shading was bound by instruction fetch: the code of one material class does
+// not fit the caches nearest the schedulers, and warps spread over classes
+// and over the code fetched it apart (28 of 55 stall cycles per issue waited
+// for instructions).  So the class-ordered queue is handed out in chunks from
+// one counter, which keeps the SM's blocks in one class at a time, and the
+// four warps of a block start each chunk together (3 of 16 stall cycles, 2.61
+// -> 1.89 ms for 1.45M rays).  With fetches shared, more registers and fewer
+// warps win: 4 blocks at 128 registers against 8 at 64 (124.3 and 125.3 ms,
+// 8 samples of the 1080p instanced scene; 30.9 and 32.8 ms, 16 samples of the
+// Cornell box).  Blocks of 256 and 512 threads: 2 % faster on the first, 2 to
+// 8 % slower on the second, which has only 3.5 chunks a block.
+constexpr int kShadeThreads = 128;
 #ifndef MT_SHADE_MIN_BLOCKS
-#define MT_SHADE_MIN_BLOCKS 8
+#define MT_SHADE_MIN_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(kStreamThreads, MT_SHADE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
     k_wf_shade(StreamView v) {
   const uint32_t cur = v.q->cur, regroup = v.q->regroup;
   if (blockIdx.x == 0) {
@@ -433,7 +451,15 @@ __global__ void __launch_bounds__(kStreamThreads, MT_SHADE_MIN_BLOCKS)
   }
   const uint32_t n = v.q->rayCount[cur];
   const uint32_t *queue = regroup ? v.sortedQueue : v.rayQueue[cur];
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+  __shared__ uint32_t taken;
+  const uint32_t chunks = (n + kShadeThreads - 1u) / kShadeThreads;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) taken = atomicAdd(&v.q->shadeNext, 1u);
+    __syncthreads();
+    if (taken >= chunks) break;
+    const uint32_t t = taken * kShadeThreads + threadIdx.x;
+    if (t >= n) continue;
     uint32_t s = queue[t];
     if (s >= v.slotCount) continue;
     Slot &sl = v.slots[s];
@@ -511,7 +537,10 @@ __global__ void __launch_bounds__(kStreamThreads, MT_SHADOW_MIN_BLOCKS) k_wf_sha
 
 __global__ void __launch_bounds__(kStreamThreads) k_wf_finish(StreamView v) {
   const uint32_t cur = v.q->cur;
-  if (blockIdx.x == 0 && threadIdx.x == 0) v.q->shadowNext = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    v.q->shadowNext = 0;
+    v.q->shadeNext = 0;
+  }
   const uint32_t n = v.q->finishCount;
   uint32_t paths = 0;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -683,12 +712,12 @@ cudaError_t carveout(const void *kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
 }
 
-cudaError_t gridFor(const void *kernel, uint32_t &grid) {
+cudaError_t gridFor(const void *kernel, uint32_t &grid, int threads = kStreamThreads) {
   int device = 0, sms = 0, perSm = 0;
   cudaError_t e = carveout(kernel);
   if (e == cudaSuccess) e = cudaGetDevice(&device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kStreamThreads, 0);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, 0);
   if (e != cudaSuccess) return e;
   grid = uint32_t(std::max(1, sms * std::max(1, perSm)));
   return cudaSuccess;
@@ -737,7 +766,7 @@ void launchIteration(const GraphKey &k, cudaStream_t s, cudaGraphConditionalHand
   else k_wf_extend<false><<<gExtend, kStreamThreads, 0, s>>>(v);
   if (k.regroupInterval) k_wf_classify<<<gRegroup, kStreamThreads, 0, s>>>(v);
   if (k.regroupInterval) k_wf_regroup<<<gRegroup, kStreamThreads, 0, s>>>(v);
-  k_wf_shade<<<gShade, kStreamThreads, 0, s>>>(v);
+  k_wf_shade<<<gShade, kShadeThreads, 0, s>>>(v);
   if (k.alpha) {
     if (k.gpuLayout) k_wf_shadow<true, true><<<gShadow, kStreamThreads, 0, s>>>(v);
     else k_wf_shadow<false, true><<<gShadow, kStreamThreads, 0, s>>>(v);
@@ -945,7 +974,7 @@ mt_status streamLaunch(const void *table, uint32_t capacity, const mtc_stream_co
   uint32_t gSeed, gExtend, gShade, gShadow, gFinish, gRegroup, gSort;
   if ((e = gridFor((const void *)k_wf_seed, gSeed)) != cudaSuccess ||
       (e = gridFor((const void *)k_wf_extend<false>, gExtend)) != cudaSuccess ||
-      (e = gridFor((const void *)k_wf_shade, gShade)) != cudaSuccess ||
+      (e = gridFor((const void *)k_wf_shade, gShade, kShadeThreads)) != cudaSuccess ||
       (e = gridFor((const void *)k_wf_shadow<false, false>, gShadow)) != cudaSuccess ||
       (e = gridFor((const void *)k_wf_finish, gFinish)) != cudaSuccess ||
       (e = gridFor((const void *)k_wf_regroup, gRegroup)) != cudaSuccess ||
