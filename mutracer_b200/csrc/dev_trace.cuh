@@ -708,21 +708,23 @@ struct RayTraversal {
     ptr = -1;
   }
 
-  // Takes entry `e` of the warp's batch, whose ray passed the root box.
-  MTD void begin(WarpRays &rays, uint32_t e, uint32_t lane, const DevScene &s, int32_t base) {
+  // Starts a query whose ray (`i` its inverse direction) passed the root box;
+  // `column` is the lane's column of its warp's world-space rays.
+  MTD void begin(const DevScene &s, int32_t base, float *column, V3 ro, V3 rd, V3 i, float limit, int32_t tri,
+                 int32_t ins, bool bothSides) {
     scene = &s; bvh = s.bvh; blasBase = base;
-    world = &rays.ray[0][lane];
-    float w[9];
+    world = column;
+    const float w[9] = {ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, i.x, i.y, i.z};
 #pragma unroll
-    for (int k = 0; k < 9; k++) world[32 * k] = w[k] = rays.pending[k][e];
-    ray.set({w[0], w[1], w[2]}, {w[6], w[7], w[8]});
-    tMax = rays.pending[9][e];
-    currentTri = __float_as_int(rays.pending[10][e]);
-    currentIns = __float_as_int(rays.pending[11][e]);
-    doubleSided = __float_as_uint(rays.pending[13][e]) >> 31;
+    for (int k = 0; k < 9; k++) world[32 * k] = w[k];
+    ray.set(ro, i);
+    tMax = limit;
+    currentTri = tri;
+    currentIns = ins;
+    doubleSided = bothSides;
     if (kAlpha) {
       alphaSmp = nullptr;
-      tMaxInit = tMax;
+      tMaxInit = limit;
     }
     bary = v3(0.0f);
     hitTri = -1; hitIns = -1;
@@ -897,27 +899,30 @@ struct RayTraversal {
   }
 };
 
-// Drains queries [0, count) of a source with the calling warp (all 32 lanes
-// call it).  The warp takes up to 32 queries at a time off the shared counter
-// `next`, every lane reading one of them, so that the chain of dependent
-// loads behind a query (counter, queue, record, scene) is paid once a batch
-// instead of by a whole warp at each lane's refill.  Where there are fewer
-// queries than lanes, the batches shrink so that every warp gets some.
+// The root box test that starts every query.
+MTD bool entersScene(const DevScene &s, V3 o, V3 inv, float limit) {
+  return intersectBox(o, xyz(ld4(s.bvh)), xyz(ld4(s.bvh + 1)), inv, limit) > 0.0f;
+}
+
+// Drains a source's queries, numbered below `end`, with the calling warp (all
+// 32 lanes call it).  The warp takes up to 32 queries at a time, every lane
+// reading one of them, so that the chain of dependent loads behind a query
+// (counter, queue, record, scene) is paid once a batch instead of by a whole
+// warp at each lane's refill.
 //
-// The source has scene(i) and blasBase(i), read(t, query): false when query t
-// is answered without a traversal, missed(query), and done(traversal,
-// payload) for a finished one, and alpha(traversal, payload, scene).
+// The source has take(n): the number of the first of n queries that no one
+// else gets; scene(i) and blasBase(i); read(t, query): false when query t is
+// answered without a traversal; missed(query) for a ray past the root box,
+// done(traversal, payload) for a finished one; and alpha(traversal, payload,
+// scene) before a shadow query with coverage starts.
 template <bool shadow, bool kGpuLayout, bool kAlpha, class Source>
-MTD void traceQueue(Source &src, uint32_t count, uint32_t *next, uint32_t refillLanes, uint32_t steps,
-                    WarpRays &rays) {
+MTD void traceQueue(Source &src, uint32_t end, uint32_t batch, uint32_t nodeLanes, uint32_t refillLanes,
+                    uint32_t steps, WarpRays &rays) {
   int2 stack[kTraversalStackEntries];
   RayTraversal<shadow, kGpuLayout, kAlpha> rt;
   rt.stack = stack;
   rt.finish(rt.kIdle);
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
-  const uint32_t batch = min(32u, max(1u, (count + warps - 1u) / warps));
-  const uint32_t nodeLanes = count / warps >= kDenseRays ? kNodeLanes : 1u;
   uint32_t payload = 0, head = 0, have = 0;
   bool exhausted = false;
   for (;;) {
@@ -926,17 +931,14 @@ MTD void traceQueue(Source &src, uint32_t count, uint32_t *next, uint32_t refill
     // Refill once enough lanes wait (or none is left tracing).
     if (uint32_t(__popc(idle)) >= refillLanes || idle == 0xffffffffu) {
       if (head == have && !exhausted) {
-        uint32_t first = 0;
-        if (lane == 0) first = atomicAdd(next, batch);
-        first = __shfl_sync(0xffffffffu, first, 0);
-        exhausted = first >= count || count - first <= batch;
+        const uint32_t first = src.take(batch);
+        exhausted = first >= end || end - first <= batch;
         RayQuery q;
-        bool keep = lane < batch && first < count && lane < count - first && src.read(first + lane, q);
+        bool keep = lane < batch && first < end && lane < end - first && src.read(first + lane, q);
         V3 inv = v3(0.0f);
         if (keep) {
-          const float4 *bvh = src.scene(q.scene).bvh;
           inv = traversalInverse(q.d);
-          if (!(intersectBox(q.o, xyz(ld4(bvh)), xyz(ld4(bvh + 1)), inv, q.limit) > 0.0f)) {
+          if (!entersScene(src.scene(q.scene), q.o, inv, q.limit)) {
             src.missed(q);
             keep = false;
           }
@@ -954,12 +956,16 @@ MTD void traceQueue(Source &src, uint32_t count, uint32_t *next, uint32_t refill
         head = 0;
         have = __popc(kept);
       }
-      const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
-      if (rt.state == rt.kIdle && head + rank < have) {
-        const uint32_t e = head + rank;
-        payload = __float_as_uint(rays.pending[12][e]);
-        const uint32_t i = __float_as_uint(rays.pending[13][e]) & 0x7fffffffu;
-        rt.begin(rays, e, lane, src.scene(i), src.blasBase(i));
+      const uint32_t e = head + __popc(idle & ((1u << lane) - 1u));
+      if (rt.state == rt.kIdle && e < have) {
+        float w[14];
+#pragma unroll
+        for (int k = 0; k < 14; k++) w[k] = rays.pending[k][e];
+        payload = __float_as_uint(w[12]);
+        const uint32_t i = __float_as_uint(w[13]) & 0x7fffffffu;
+        rt.begin(src.scene(i), src.blasBase(i), &rays.ray[0][lane], {w[0], w[1], w[2]}, {w[3], w[4], w[5]},
+                 {w[6], w[7], w[8]}, w[9], __float_as_int(w[10]), __float_as_int(w[11]),
+                 __float_as_uint(w[13]) >> 31);
         if (kAlpha) src.alpha(rt, payload, i);
       }
       __syncwarp();

@@ -84,28 +84,69 @@ __global__ void k_sample_maps(const __grid_constant__ DevScene s, const int32_t 
   out[i] = sampleMap(s, indices[i], V2{uv.x, uv.y});
 }
 
-template <bool kGpuLayout>
-__global__ void k_first_hit(const __grid_constant__ DevScene s, int32_t blasBase, int32_t isEmpty, const float4 *rays,
-                            uint32_t count, mtc_hit *hits) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  float4 o4 = rays[size_t(i) * 2], d4 = rays[size_t(i) * 2 + 1];
-  mtc_hit out;
-  out.hit = 0; out.instance = -1; out.record = -1; out.t = RAY_MAX_DISTANCE;
-  out.barycentric[0] = 0; out.barycentric[1] = 0; out.barycentric[2] = 0; out._pad = 0;
-  if (!isEmpty) {
-    TraversalHit h;
-    h.tMax = RAY_MAX_DISTANCE;
-    h.triangleIndex = -1;
-    h.insIdx = -1;
-    h.hitBary = v3(0.0f);
-    traverse<false, kGpuLayout>(s, blasBase, xyz(o4), xyz(d4), 0, false, -1, -1, h);
-    if (h.insIdx >= 0) {
-      out.hit = 1; out.instance = h.insIdx; out.record = h.triangleIndex; out.t = h.tMax;
-      out.barycentric[0] = h.hitBary.x; out.barycentric[1] = h.hitBary.y; out.barycentric[2] = h.hitBary.z;
-    }
+// querySceneSoftware for `raysPerWarp` consecutive rays a warp, through the
+// traversal of the wavefront engine: a lane whose ray is finished takes the
+// warp's next one.  Latency- and divergence-bound: 1M scattered rays over the
+// 4M-triangle instanced scene take 2.80 ms, with one ray a thread for good
+// 5.56 ms; 33 rays 17 us against 24 us, launch included.
+struct FirstHitSource {
+  const DevScene &s;
+  const float4 *rays;
+  mtc_hit *hits;
+  int32_t base;
+  bool empty;
+  uint32_t cursor;
+  MTD uint32_t take(uint32_t n) {
+    const uint32_t first = cursor;
+    cursor += n;
+    return first;
   }
-  hits[i] = out;
+  MTD const DevScene &scene(uint32_t) const { return s; }
+  MTD int32_t blasBase(uint32_t) const { return base; }
+  MTD bool read(uint32_t t, RayQuery &q) const {
+    q.payload = t;
+    if (empty) {
+      missed(q);
+      return false;
+    }
+    q.o = xyz(rays[size_t(t) * 2]);
+    q.d = xyz(rays[size_t(t) * 2 + 1]);
+    q.limit = RAY_MAX_DISTANCE;
+    q.tri = -1;
+    q.ins = -1;
+    q.scene = 0;
+    q.doubleSided = false;
+    return true;
+  }
+  MTD void missed(const RayQuery &q) const {
+    mtc_hit out;
+    out.hit = 0; out.instance = -1; out.record = -1; out.t = RAY_MAX_DISTANCE;
+    out.barycentric[0] = 0; out.barycentric[1] = 0; out.barycentric[2] = 0; out._pad = 0;
+    hits[q.payload] = out;
+  }
+  template <class T>
+  MTD void done(const T &rt, uint32_t t) const {
+    mtc_hit out;
+    out.hit = rt.found() ? 1 : 0; out.instance = rt.hitIns; out.record = rt.hitTri; out.t = rt.tMax;
+    out.barycentric[0] = rt.bary.x; out.barycentric[1] = rt.bary.y; out.barycentric[2] = rt.bary.z; out._pad = 0;
+    hits[t] = out;
+  }
+  template <class T>
+  MTD void alpha(T &, uint32_t, uint32_t) const {}
+};
+
+constexpr int kHitThreads = 128;
+template <bool kGpuLayout>
+__global__ void __launch_bounds__(kHitThreads, 5)
+    k_first_hit(const __grid_constant__ DevScene s, int32_t blasBase, int32_t isEmpty, const float4 *rays,
+                uint32_t count, uint32_t raysPerWarp, mtc_hit *hits) {
+  __shared__ WarpRays warpRays[kHitThreads / 32];
+  const uint64_t first = (uint64_t(blockIdx.x) * (kHitThreads / 32) + threadIdx.x / 32u) * raysPerWarp;
+  if (first >= count) return;
+  const uint32_t end = uint32_t(min(uint64_t(count), first + raysPerWarp));
+  FirstHitSource src{s, rays, hits, blasBase, isEmpty != 0, uint32_t(first)};
+  traceQueue<false, kGpuLayout, false>(src, end, min(32u, raysPerWarp), raysPerWarp >= kDenseRays ? kNodeLanes : 1u,
+                                       4u, 8u, warpRays[threadIdx.x / 32u]);
 }
 
 // read_average (native/host/src/lib.rs:343-364): each f32 of an accumulation
@@ -263,13 +304,19 @@ mt_status mtc_query_first_hit(const mtc_scene_view *scene, const float *rays, ui
                               void *stream) {
   if (!validScene(scene) || (!rays && count) || (!hits && count)) return MT_ERROR_INVALID_ARGUMENT;
   if (count == 0) return MT_OK;
-  int32_t blasBase = scene->blas_offset;
-  if (scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT)
-    k_first_hit<true><<<(count + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-        toDev(scene), blasBase, scene->instance_count == 0, (const float4 *)rays, count, hits);
-  else
-    k_first_hit<false><<<(count + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-        toDev(scene), blasBase, scene->instance_count == 0, (const float4 *)rays, count, hits);
+  int device = 0, sms = 148;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  // A few rays: one a warp, which then waits for no other.  Many: up to 256 a
+  // warp, as long as there are enough warps left to fill the SMs three times.
+  const uint64_t warps = uint64_t(sms) * 5u * (kHitThreads / 32) * 3u;
+  const uint32_t perWarp = uint32_t(std::min<uint64_t>(256u, (count + warps - 1u) / warps));
+  const uint32_t perBlock = perWarp * (kHitThreads / 32);
+  const uint32_t grid = uint32_t((uint64_t(count) + perBlock - 1u) / perBlock);
+  const int32_t blasBase = scene->blas_offset;
+  auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_first_hit<true> : k_first_hit<false>;
+  kernel<<<grid, kHitThreads, 0, (cudaStream_t)stream>>>(toDev(scene), blasBase, scene->instance_count == 0,
+                                                         (const float4 *)rays, count, perWarp, hits);
   return cudaStatus(cudaGetLastError());
 }
 

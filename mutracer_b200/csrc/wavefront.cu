@@ -272,11 +272,31 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_seed(StreamView v, uint32
 #ifndef MT_SHADOW_MIN_BLOCKS
 #define MT_SHADOW_MIN_BLOCKS 6
 #endif
+// Drains a queue of `count` rays behind the counter `next` with every warp of
+// the grid.  Where there are fewer rays than lanes, the batches shrink so
+// that every warp gets some.
+template <bool shadow, bool kGpuLayout, bool kAlpha, class Source>
+MTD void drainQueue(const StreamView &v, Source &src, uint32_t count) {
+  __shared__ WarpRays rays[kStreamThreads / 32];
+  const uint32_t warps = gridDim.x * (kStreamThreads / 32);
+  const uint32_t batch = min(32u, max(1u, (count + warps - 1u) / warps));
+  traceQueue<shadow, kGpuLayout, kAlpha>(src, count, batch, count / warps >= kDenseRays ? kNodeLanes : 1u,
+                                         v.refillLanes, v.stepsPerCheck, rays[threadIdx.x / 32u]);
+}
+
+// A warp's next n entries behind a shared counter.
+MTD uint32_t takeBatch(uint32_t *next, uint32_t n) {
+  uint32_t first = 0;
+  if (laneId() == 0) first = atomicAdd(next, n);
+  return __shfl_sync(0xffffffffu, first, 0);
+}
+
 // The extension rays of one event iteration.
 struct ExtendSource {
   const StreamView &v;
   const uint32_t *queue;
   uint32_t rays;
+  MTD uint32_t take(uint32_t n) const { return takeBatch(&v.q->extendNext, n); }
   MTD const DevScene &scene(uint32_t job) const { return v.jobs[job].s; }
   MTD int32_t blasBase(uint32_t job) const { return v.jobs[job].u.blas_offset; }
   MTD void store(uint32_t s, float t, V3 bary, int32_t tri, int32_t ins) const {
@@ -318,7 +338,6 @@ struct ExtendSource {
 template <bool kGpuLayout>
 __global__ void __launch_bounds__(kStreamThreads, MT_EXTEND_MIN_BLOCKS)
     k_wf_extend(StreamView v) {
-  __shared__ WarpRays rays[kStreamThreads / 32];
   const uint32_t cur = v.q->cur;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     v.q->rayCount[cur ^ 1u] = 0;
@@ -334,8 +353,7 @@ __global__ void __launch_bounds__(kStreamThreads, MT_EXTEND_MIN_BLOCKS)
     }
   }
   ExtendSource src{v, v.sortRays ? v.sortedRays : v.rayQueue[cur], 0u};
-  traceQueue<false, kGpuLayout, false>(src, n, &v.q->extendNext, v.refillLanes, v.stepsPerCheck,
-                                       rays[threadIdx.x / 32u]);
+  drainQueue<false, kGpuLayout, false>(v, src, n);
   flush(v, src.rays, 0, 0);
 }
 
@@ -497,6 +515,7 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
 struct ShadowSource {
   const StreamView &v;
   uint32_t rays;
+  MTD uint32_t take(uint32_t n) const { return takeBatch(&v.q->shadowNext, n); }
   MTD const DevScene &scene(uint32_t job) const { return v.jobs[job].s; }
   MTD int32_t blasBase(uint32_t job) const { return v.jobs[job].u.blas_offset; }
   MTD bool read(uint32_t t, RayQuery &q) {
@@ -528,10 +547,8 @@ struct ShadowSource {
 
 template <bool kGpuLayout, bool kAlpha>
 __global__ void __launch_bounds__(kStreamThreads, MT_SHADOW_MIN_BLOCKS) k_wf_shadow(StreamView v) {
-  __shared__ WarpRays rays[kStreamThreads / 32];
   ShadowSource src{v, 0u};
-  traceQueue<true, kGpuLayout, kAlpha>(src, v.q->shadowCount, &v.q->shadowNext, v.refillLanes, v.stepsPerCheck,
-                                       rays[threadIdx.x / 32u]);
+  drainQueue<true, kGpuLayout, kAlpha>(v, src, v.q->shadowCount);
   flush(v, 0, src.rays, 0);
 }
 
