@@ -236,12 +236,11 @@ class StreamBatch(_JobTable):
 
 
 # Launch shapes the autotuner tries, in BatchConfig.make's order (block
-# threads, warp tile width, CTAs per SM, items per fetch).  The kernel is
-# compiled for 16 resident 128-thread CTAs per SM (32 registers), so 16 fills
-# the SMs; larger grids only queue CTAs behind them.
+# threads, warp tile width, CTAs per SM, items per fetch).  0 keeps the default:
+# one block an SM, all its warps in step; smaller blocks share less of the code
+# they fetch.
 AUTOTUNE_SPACE = (
-    (128, 8, 16, 1), (128, 8, 16, 2), (128, 4, 16, 1), (128, 16, 16, 1),
-    (128, 32, 16, 1), (64, 8, 32, 1), (128, 8, 8, 1), (128, 8, 12, 1),
+    (0, 8, 0, 1), (0, 8, 0, 2), (0, 4, 0, 1), (0, 16, 0, 1), (0, 32, 0, 1), (128, 8, 8, 1), (128, 8, 4, 1),
 )
 
 

@@ -109,12 +109,11 @@ inline JobData makeJob(const mtc_scene_view *scene, const mtc_camera_uniform *ca
   return J;
 }
 
-// Resident CTAs of 128 threads per SM the persistent batched kernels are
-// compiled for (32 registers; the default grid fills them): like the plain
-// kernel, latency-bound, so more warps beat fewer spills.
-#ifndef MT_BATCH_MIN_BLOCKS
-#define MT_BATCH_MIN_BLOCKS 16
-#endif
+// Threads per block the megakernels are compiled for and run with by default:
+// one block fills an SM at 64 registers, its 32 warps in step (tracePixels).
+// 512 threads at 128 registers: 20 % faster on glass and on 256x256 previews,
+// 10 to 30 % slower on the Cornell, instanced and batched runs.
+constexpr uint32_t kPixelThreads = 1024;
 
 struct BatchShape {
   uint32_t blockThreads, tileW, tileH, ctasPerSm, grain;
@@ -122,7 +121,7 @@ struct BatchShape {
 // Resolves a (possibly NULL) mtc_batch_config to launch parameters; false for
 // out-of-range values.
 inline bool batchShape(const mtc_batch_config *c, BatchShape &out) {
-  out = BatchShape{128u, 8u, 4u, uint32_t(MT_BATCH_MIN_BLOCKS), 1u};
+  out = BatchShape{kPixelThreads, 8u, 4u, 1u, 1u};
   if (!c) return true;
   if (c->struct_size != sizeof(mtc_batch_config)) return false;
   if (c->block_threads) {
@@ -134,6 +133,7 @@ inline bool batchShape(const mtc_batch_config *c, BatchShape &out) {
     out.tileW = c->tile_width;
     out.tileH = 32u / c->tile_width;
   }
+  out.ctasPerSm = kPixelThreads / out.blockThreads;
   if (c->ctas_per_sm) {
     if (c->ctas_per_sm > 32u) return false;
     out.ctasPerSm = c->ctas_per_sm;
@@ -174,46 +174,76 @@ inline mt_status writeBatchTable(const mtc_job_desc *jobs, uint32_t job_count, c
   return MT_OK;
 }
 
-// The persistent work loop of the batched kernels.  queue[0] is the next
-// work item; items are warp tiles (tileW x 32/tileW pixels) laid out job
-// after job (JobData.firstItem / .items).  A warp takes `grain` consecutive
-// items per atomic and runs every sample of each tile's pixels in order.
-// The loop ends when the counter passes the item total, so every warp exits;
-// its iteration bound only guards against a corrupted table, and running
-// out of it sets kBatchStatusGuardExhausted in `status` (when given).
+// The pixels of a job table, claimed by the lanes of a persistent grid.
+// queue[0] is the next work item; items are warp tiles (tileW x 32/tileW
+// pixels) laid out job after job (JobData.firstItem / .items).  A warp takes
+// `grain` consecutive items per atomic and hands their pixels to its lanes as
+// they ask.  A warp is done when the counter passes the item total; its fetch
+// bound only guards against a corrupted table, and running out of it sets
+// kBatchStatusGuardExhausted in `status` (when given).
+struct TableClaims {
+  const BatchHeader *header;
+  const JobData *jobs;
+  uint32_t *queue;
+  uint32_t *status;
+  uint32_t grain;
+  uint64_t cursor = 0, end = 0;  // units (pixels of the tiles taken) left
+  uint32_t fetches = 0;
+  bool exhausted = false;
+
+  MTD TableClaims(const BatchHeader *h, uint32_t *q, uint32_t *st, uint32_t g)
+      : header(h), jobs(reinterpret_cast<const JobData *>(reinterpret_cast<const char *>(h) + kBatchTableOffset)),
+        queue(q), status(st), grain(g) {}
+
+  MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &samples) {
+    const uint32_t lane = threadIdx.x & 31u, total = header->totalItems, tileW = header->tileW;
+    unsigned asking = __ballot_sync(0xffffffffu, wants);
+    while (asking && !exhausted) {
+      if (cursor == end) {
+        uint32_t first = 0;
+        if (lane == 0) first = atomicAdd(queue, grain);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (first >= total || fetches++ > total) {
+          if (first < total && status && lane == 0) atomicOr(status, kBatchStatusGuardExhausted);
+          exhausted = true;
+          break;
+        }
+        cursor = uint64_t(first) * 32u;
+        end = uint64_t(min(first + grain, total)) * 32u;
+      }
+      const uint64_t u = cursor + __popc(asking & ((1u << lane) - 1u));
+      cursor = min(end, cursor + uint64_t(__popc(asking)));
+      if (wants && u < end) {
+        const uint32_t item = uint32_t(u / 32u), in = uint32_t(u % 32u);
+        // The job owning the item: firstItem ascends.
+        uint32_t lo = 0, hi = header->jobCount;
+        while (hi - lo > 1u) {
+          const uint32_t mid = (lo + hi) / 2u;
+          if (jobs[mid].firstItem <= item) lo = mid; else hi = mid;
+        }
+        const JobData &J = jobs[lo];
+        const uint32_t local = item - J.firstItem;
+        x = (local % J.tilesX) * tileW + in % tileW;
+        y = (local / J.tilesX) * (32u / tileW) + in / tileW;
+        if (x < J.width && y < J.height && J.samples) {
+          job = &J;
+          samples = J.samples;
+          wants = false;
+        }
+      }
+      __syncwarp();
+      asking = __ballot_sync(0xffffffffu, wants);
+    }
+  }
+};
+
+// The persistent work loop of the batched kernels.
 template <bool kGpuLayout>
 __device__ __forceinline__ void batchWorkLoop(const BatchHeader *__restrict__ header, uint32_t *queue, uint32_t grain,
                                               uint32_t *status, Counters &cnt, uint32_t &paths) {
-  const JobData *__restrict__ jobs =
-      reinterpret_cast<const JobData *>(reinterpret_cast<const char *>(header) + kBatchTableOffset);
-  const uint32_t job_count = header->jobCount, total_items = header->totalItems, tileW = header->tileW;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lx = lane % tileW, ly = lane / tileW, tileH = 32u / tileW;
-  bool done = false;
-  for (uint32_t guard = 0; guard < total_items + 1u; guard++) {
-    uint32_t first = 0;
-    if (lane == 0) first = atomicAdd(queue, grain);
-    first = __shfl_sync(0xffffffffu, first, 0);
-    if (first >= total_items) {
-      done = true;
-      break;
-    }
-    const uint32_t last = min(first + grain, total_items);
-    uint32_t j = 0;
-    for (uint32_t item = first; item < last; item++) {
-      // Jobs are few; a forward scan of the prefix table finds the owner.
-      while (j + 1 < job_count && jobs[j + 1].firstItem <= item) j++;
-      const JobData &J = jobs[j];
-      uint32_t local = item - J.firstItem;
-      uint32_t tx = local % J.tilesX, ty = local / J.tilesX;
-      uint32_t x = tx * tileW + lx, y = ty * tileH + ly;
-      if (x < J.width && y < J.height) {
-        tracePixelSamples<kGpuLayout>(J, x, y, J.samples, cnt);
-        paths += J.samples;
-      }
-    }
-  }
-  if (!done && status && lane == 0) atomicOr(status, kBatchStatusGuardExhausted);
+  __shared__ float columns[kPixelThreads / 32][9 * 32];
+  TableClaims claims(header, queue, status, grain);
+  tracePixels<kGpuLayout>(claims, cnt, paths, &columns[threadIdx.x / 32u][threadIdx.x & 31u]);
 }
 
 }  // namespace mt

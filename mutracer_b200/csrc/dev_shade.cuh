@@ -830,20 +830,6 @@ MTD void completeSurfaceInteraction(const JobData &J, SurfaceInteraction &si, Su
   si.position = mat4v(l0, l1, l2, l3, position, 1.0f);
 }
 
-// intersect.wgsl.ts:829-879; scenes with alpha test each candidate's
-// coverage with the path's sampler.
-template <bool kGpuLayout>
-MTD bool intersectSceneShadow(const JobData &J, const Ray &r, float lightDistance, int32_t tri, int32_t ins,
-                              Counters &cnt, Sampler &smp) {
-  if (J.u.is_empty > 0) return false;
-  cnt.shadow++;
-  TraversalHit h;
-  h.tMax = fminf(fmaxf(lightDistance, 0.0f), RAY_MAX_DISTANCE);
-  if (J.s.flags & MTC_SCENE_HAS_ALPHA)
-    return traverse<true, kGpuLayout, true>(J.s, J.u.blas_offset, r.o, r.d, 1, true, tri, ins, h, &smp);
-  return traverse<true, kGpuLayout>(J.s, J.u.blas_offset, r.o, r.d, 1, true, tri, ins, h);
-}
-
 // ------------------------------------------------------------- integrator
 struct Path {
   bool scatteringMediumEntered;
@@ -1447,18 +1433,6 @@ MTD bool reusesPrimary(const JobData &J, const PathSample &ps, bool primaryReady
   return isSpectral(J) && ps.event == 0 && primaryReady;
 }
 
-template <bool kGpuLayout>
-MTD void traceExtension(const JobData &J, const PathSample &ps, TraversalHit &h, Counters &cnt) {
-  h.tMax = RAY_MAX_DISTANCE;
-  h.triangleIndex = -1;
-  h.insIdx = -1;
-  if (J.u.is_empty > 0) return;
-  cnt.ext++;
-  traverse<false, kGpuLayout>(J.s, J.u.blas_offset, ps.path.ray.o, ps.path.ray.d, ps.depth, ps.event != 0,
-                              ps.si.triangleIndex,
-                  ps.si.instanceIndex, h);
-}
-
 // The rest of one iteration of the integrator's event loop
 // (rayTrace.compute.ts:906-944) once the extension ray's closest hit `h` is
 // known: surface interaction, material, primary guides or completeVertex,
@@ -1774,29 +1748,40 @@ MTD bool finishWavelength(const JobData &J, PathSample &ps, SpectralState &sp) {
   return false;
 }
 
-// One iteration of the integrator's event loop: true when the path (the
-// current wavelength path of a spectral sample) has ended.
-template <bool kGpuLayout>
-MTD bool stepPath(Ctx &c, PathSample &ps, SpectralState &sp) {
-  TraversalHit h;
-  h.tMax = RAY_MAX_DISTANCE;
-  h.triangleIndex = -1;
-  h.insIdx = -1;
-  const bool spectral = isSpectral(c.J), split = alphaSplit(c.J);
-  const bool reuse = spectral ? reusesPrimary(c.J, ps, sp.primaryReady) : split && sp.frontPending;
-  if (!reuse) traceExtension<kGpuLayout>(c.J, ps, h, c.cnt);
-  return spectral ? shadeStepSpectral(c, ps, sp, h) : split ? shadeStepAlpha(c, ps, sp, h) : shadeStep(c, ps, sp, h);
-}
-
-// The deferred NEE visibility test of sampleScattering (sampleMaterial.wgsl.ts
-// :238-245): unoccluded -> the selected candidate's contribution.
-template <bool kGpuLayout>
-MTD void resolveShadow(Ctx &c, PathSample &ps) {
-  if (!c.shadow.valid) return;
-  c.shadow.valid = false;
-  if (!intersectSceneShadow<kGpuLayout>(c.J, c.shadow.ray, c.shadow.maxDistance, c.shadow.triangleIndex,
-                                        c.shadow.instanceIndex, c.cnt, c.smp))
-    ps.path.li += c.shadow.contribution;
+// One query per lane of a converged warp (all 32 lanes call it; those without
+// `active` only keep the others company, their arguments unread): the closest
+// hit in `h`, or for shadow queries whether something occludes.  Out of line,
+// with the traversal's own registers: the callers' path state would spill
+// them.
+template <bool shadow, bool kGpuLayout, bool kAlpha = false>
+static __device__ __noinline__ bool traceWarp(const JobData *job, bool active, const Ray &query, bool doubleSided,
+                                              int32_t currentTri, int32_t currentIns, TraversalHit &h, float *column,
+                                              Sampler *alphaSmp) {
+  int2 stack[kTraversalStackEntries];
+  RayTraversal<shadow, kGpuLayout, kAlpha> rt;
+  rt.stack = stack;
+  rt.hitTri = -1;
+  rt.finish(rt.kIdle);
+  if (active) {
+    const V3 inv = traversalInverse(query.d);
+    if (entersScene(job->s, query.o, inv, h.tMax)) {
+      rt.begin(job->s, job->u.blas_offset, column, query.o, query.d, inv, h.tMax, currentTri, currentIns, doubleSided);
+      if (kAlpha) rt.alphaSmp = alphaSmp;
+    }
+  }
+  __syncwarp();
+  // Each lane has this one ray: one node visit a round keeps the lanes at
+  // leaves and instances moving (58.8 against 64.5 ms with visits repeated
+  // while 12 lanes need one, 4 samples of the instanced scene at 960x540).
+  while (__any_sync(0xffffffffu, rt.state < rt.kDone)) rt.advance(1u, 1u);
+  if (!shadow && rt.found()) {
+    h.tMax = rt.tMax;
+    h.hitBary = rt.bary;
+    h.triangleIndex = rt.hitTri;
+    h.insIdx = rt.hitIns;
+    h.hitNormal = hitNormal(job->s, rt.hitTri, rt.hitIns);
+  }
+  return rt.found();
 }
 
 // rayTrace.compute.ts:1209-1262: clamp, NaN guard and accumulation of the
@@ -1824,45 +1809,90 @@ static __device__ __noinline__ void endSample(const JobData &J, uint32_t idx, co
   *mom = make_float4(m.x + lum, m.y + lum * lum, m.z, m.w);
 }
 
-// `samples` consecutive progressive passes of pixel (x, y), in order, each
-// accumulated before the next begins (the same sums as `samples` separate
-// dispatches).  The thread runs its own sample sequence in one event loop,
-// so a lane whose path ended early starts its next sample while the warp's
-// longer paths are still tracing.  Kept out of line so that every kernel that
-// traces pixels (plain, batched, allocation-free batched) calls the same
-// out-of-line function, compiled once per translation unit from this one
-// source, instead of an inlined copy shaped by its caller: inlined copies could
-// contract multiply-adds differently, and a job's image must be bit-identical
-// alone and in a batch.
-template <bool kGpuLayout>
-static __device__ __noinline__ void tracePixelSamples(const JobData &J, uint32_t x, uint32_t y, uint32_t samples,
-                                                      Counters &cnt) {
-  Ctx c{J, Sampler(), BsdfContext{J.s.lut, (J.s.flags & MTC_SCENE_HAS_MEDIUM) != 0u, feature(J, MTC_FEATURE_HAS_THIN_FILM)},
-        Counters(), ShadowQuery()};
-  c.shadow.valid = false;
-  const uint32_t idx = x + y * J.width;
+// The megakernels' work loop, run by all threads of a block together.  Each
+// lane owns a pixel of a job at a time: all its samples in order, each
+// accumulated before the next begins (the same sums as as many separate
+// dispatches), then the next pixel that `claims` gives it.  `column` is the
+// lane's column of its warp's world-space rays in shared memory.
+//
+// Instruction fetch is what bounds these kernels once each warp runs on its
+// own: 64 warps an SM at different places of the shading code fetch it apart.
+// So the whole block traces its extension rays, meets, and shades, one event
+// at a time: the 32 warps of one 1,024-thread block an SM share what they
+// fetch (figures at k_trace).  Lanes stay busy by claiming pixels one by one.
+//
+// claims.next(wants, job, x, y, samples), called by whole warps, gives a lane
+// that wants one its next pixel with samples to add (samples stays 0: none is
+// left).
+template <bool kGpuLayout, class Claims>
+MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths, float *column) {
+  // A job's Ctx is made anew at each claim; it is only used while left > 0.
+  alignas(16) unsigned char room[sizeof(Ctx)];
+  Ctx &c = *reinterpret_cast<Ctx *>(room);
+  const JobData *job = nullptr;
   PathSample ps;
   SpectralState sp;
-  const bool spectral = isSpectral(J), split = alphaSplit(J);
-  uint32_t left = samples;
-  bool active = left > 0u;
-  if (active) beginSample(c, x, y, ps, sp);
-  // No warp vote here: the traversal and shading are latency-bound, and
-  // lanes left free to diverge give the scheduler more independent loads in
-  // flight than a warp forced back together at every event.
-  while (active) {
-    bool ended = stepPath<kGpuLayout>(c, ps, sp);
-    resolveShadow<kGpuLayout>(c, ps);
-    if (ended && spectral) ended = finishWavelength(J, ps, sp);
-    else if (ended && split) ended = finishAlphaSplit(J, ps, sp);
-    if (ended) {
-      endSample(J, idx, ps);
-      if (--left == 0u) active = false;
-      else beginSample(c, x, y, ps, sp);
+  uint32_t x = 0, y = 0, left = 0;
+  for (;;) {
+    const bool wants = left == 0u;
+    claims.next(wants, job, x, y, left);
+    if (wants && left) {
+      paths += left;
+      new (room) Ctx{*job, Sampler(),
+                     BsdfContext{job->s.lut, (job->s.flags & MTC_SCENE_HAS_MEDIUM) != 0u,
+                                 feature(*job, MTC_FEATURE_HAS_THIN_FILM)},
+                     Counters(), ShadowQuery()};
+      beginSample(c, x, y, ps, sp);
     }
+    const bool active = left != 0u;
+    if (!__syncthreads_or(active)) break;
+    bool spectral = false, split = false, extend = false, alpha = false, ended = false, query = false;
+    TraversalHit h;
+    h.tMax = RAY_MAX_DISTANCE;
+    h.triangleIndex = -1;
+    h.insIdx = -1;
+    if (active) {
+      spectral = isSpectral(*job);
+      split = alphaSplit(*job);
+      alpha = (job->s.flags & MTC_SCENE_HAS_ALPHA) != 0u;
+      // The extension ray of the path's event, but for a path that restarts
+      // at its primary vertex.
+      extend = !(job->u.is_empty > 0) &&
+               !(spectral ? reusesPrimary(*job, ps, sp.primaryReady) : split && sp.frontPending);
+      if (extend) cnt.ext++;
+    }
+    traceWarp<false, kGpuLayout>(job, extend, ps.path.ray, ps.event != 0, ps.depth > 0 ? ps.si.triangleIndex : -1,
+                                 ps.si.instanceIndex, h, column, nullptr);
+    __syncthreads();
+    if (active) {
+      c.shadow.valid = false;
+      ended = spectral ? shadeStepSpectral(c, ps, sp, h) : split ? shadeStepAlpha(c, ps, sp, h) : shadeStep(c, ps, sp, h);
+      query = c.shadow.valid;
+    }
+    __syncwarp();
+    // The deferred NEE visibility test of sampleScattering
+    // (sampleMaterial.wgsl.ts:238-245): unoccluded -> the selected
+    // candidate's contribution.
+    if (__any_sync(0xffffffffu, query)) {
+      const bool trace = query && !(job->u.is_empty > 0);
+      if (trace) cnt.shadow++;
+      if (query) h.tMax = fminf(fmaxf(c.shadow.maxDistance, 0.0f), RAY_MAX_DISTANCE);
+      const bool occluded =
+          __any_sync(0xffffffffu, query && alpha)
+              ? traceWarp<true, kGpuLayout, true>(job, trace, c.shadow.ray, true, c.shadow.triangleIndex,
+                                                  c.shadow.instanceIndex, h, column, alpha ? &c.smp : nullptr)
+              : traceWarp<true, kGpuLayout>(job, trace, c.shadow.ray, true, c.shadow.triangleIndex,
+                                            c.shadow.instanceIndex, h, column, nullptr);
+      if (query && !occluded) ps.path.li += c.shadow.contribution;
+    }
+    if (ended && spectral) ended = finishWavelength(*job, ps, sp);
+    else if (ended && split) ended = finishAlphaSplit(*job, ps, sp);
+    if (ended) {
+      endSample(*job, x + y * job->width, ps);
+      if (--left) beginSample(c, x, y, ps, sp);
+    }
+    __syncwarp();
   }
-  cnt.ext += c.cnt.ext;
-  cnt.shadow += c.cnt.shadow;
 }
 
 }  // namespace mt

@@ -341,188 +341,6 @@ struct TraversalHit {
   int32_t triangleIndex, insIdx;
 };
 
-// Levels of the near path taken in one interior visit beyond the first.
-#ifndef MT_FUSED_LEVELS
-#define MT_FUSED_LEVELS 1
-#endif
-
-// The interior visit of getBVHTraverseCode at either level (intersect.wgsl.ts
-// :265-300, :439-624 for BVH2): box-test both children (boxes given), push
-// the nearer last (the `>` rule).  The node the reference pops next is the
-// child pushed last; when that child is an interior node (its header word
-// came with its box) its children are tested in the same visit instead of
-// going through the stack, for up to MT_FUSED_LEVELS more levels.  Nothing in
-// between could change tMax, so the boxes tested, their order and the stack
-// contents are those of one level per visit.  `base` is where node indices
-// start in the buffer (the BLAS base), `rightOffset` what a right pointer is
-// relative to (the BLAS offset; 0 in the TLAS).
-MTD void visitInterior(const float4 *bvh, int32_t base, int32_t rightOffset, bool fusable, V3 ro, V3 invDir,
-                       float tMax, int32_t left, int32_t right, float4 lmin, float4 lmax, float4 rmin, float4 rmax,
-                       int32_t *stack, int &top) {
-  for (int level = 0;; level++) {
-    const float d0 = intersectBox(ro, xyz(lmin), xyz(lmax), invDir, tMax);
-    const float d1 = intersectBox(ro, xyz(rmin), xyz(rmax), invDir, tMax);
-    int32_t first = right, second = left;
-    float df = d1, ds = d0;
-    float firstPtr = rmin.w, secondPtr = lmin.w;
-    if (d0 > d1) {
-      first = left; second = right;
-      df = d0; ds = d1;
-      firstPtr = lmin.w; secondPtr = rmin.w;
-    }
-    const bool pushFirst = df > 0.0f && top + 1 < MTC_MAX_STACK;
-    const bool pushSecond = ds > 0.0f && top + (pushFirst ? 2 : 1) < MTC_MAX_STACK;
-    // The node popped next: the second child if pushed, else the first.
-    const int32_t next = pushSecond ? second : first;
-    const int32_t nextPtr = asi(pushSecond ? secondPtr : firstPtr);
-    const bool fuse = fusable && level < MT_FUSED_LEVELS && (pushFirst || pushSecond) && nextPtr >= 0;
-    if (pushFirst && !(fuse && !pushSecond)) stack[++top] = first;
-    if (pushSecond && !fuse) stack[++top] = second;
-    if (!fuse) return;
-    left = next + 2;
-    right = nextPtr + rightOffset;
-    lmin = ld4(bvh + left + base);
-    lmax = ld4(bvh + left + 1 + base);
-    rmin = ld4(bvh + right + base);
-    rmax = ld4(bvh + right + 1 + base);
-  }
-}
-
-// getBVHTraverseCode, intersect.wgsl.ts:213-629 for the BVH2 layout.  With
-// `shadow` the first accepted hit ends the query (returns true).
-//
-// kGpuLayout mirrors the reference's blasLayoutMask specialisation
-// (getBVHTraverseCode's layout branches are compiled only for the layouts a
-// scene uses): without it only BVH2 (layout 0) BLASes are traversed and the
-// BVH_GPU (layout 2) code is not compiled in.
-//
-// A shadow query with kAlpha tests each candidate hit's coverage
-// (alphaPasses, drawing from `alphaSmp`): a hit that does not occlude
-// restores the query's tMax and traversal goes on (intersect.wgsl.ts
-// :846-866).  Without kAlpha the test is not compiled in.
-template <bool shadow, bool kGpuLayout, bool kAlpha = false>
-__device__ __noinline__ bool traverse(const DevScene &s, int32_t blasBase, V3 rayO, V3 rayD, int bounces,
-                                      bool doubleSided, int32_t currentTri, int32_t currentIns, TraversalHit &h,
-                                      Sampler *alphaSmp = nullptr) {
-  const float tMaxInit = h.tMax;
-  int32_t tlasStack[MTC_MAX_STACK];
-  int32_t blasStack[MTC_MAX_STACK];
-  int tlasTop = -1;
-  const float4 *bvh = s.bvh;
-  V3 invD = traversalInverse(rayD);
-  if (intersectBox(rayO, xyz(ld4(bvh)), xyz(ld4(bvh + 1)), invD, h.tMax) > 0.0f) {
-    tlasTop = 0;
-    tlasStack[0] = 0;
-  }
-  while (tlasTop >= 0) {
-    int32_t tlasNode = tlasStack[tlasTop--];
-    float4 r1 = ld4(bvh + tlasNode);
-    int32_t ptr = asi(r1.w);
-    if (ptr >= 0) {
-      int32_t left = tlasNode + 2, right = ptr;
-      visitInterior(bvh, 0, 0, true, rayO, invD, h.tMax, left, right, ld4(bvh + left), ld4(bvh + left + 1),
-                    ld4(bvh + right), ld4(bvh + right + 1), tlasStack, tlasTop);
-      continue;
-    }
-    int32_t tlasCount = -ptr;
-    for (int32_t io = tlasCount - 1; io >= 0; io--) {
-      float4 rec = ld4(bvh + tlasNode + 2 + io);
-      int32_t insIdx = asi(rec.x);
-      int32_t blasRoot = asi(rec.y);
-      const float4 *insv = s.ins + size_t(insIdx) * MTC_INSTANCE_VEC4_STRIDE;
-      float4 insData = ld4(insv);
-      float4 c0 = ld4(insv + 1), c1 = ld4(insv + 2), c2 = ld4(insv + 3), c3 = ld4(insv + 4);
-      V3 o = xmat4(c0, c1, c2, c3, rayO, 1.0f);
-      V3 d = xmat4(c0, c1, c2, c3, rayD, 0.0f);
-      V3 linvD = traversalInverse(d);
-      int maxDim = maxDimension(vabs(d));
-      V3 shear = getShear(d, maxDim);
-      uint32_t encoded = asu(insData.x);
-      const uint32_t layout = encoded >> 30;
-      if (layout != 0u && !(kGpuLayout && layout == 2u)) continue;  // TinyBVH bvh4 / cwbvh are not consumed
-      int32_t blasOffset = int32_t(encoded & 0x3fffffffu);
-      int32_t vertexOffset = asi(insData.y);
-      int32_t sideMaterial = asi(insData.z) >> 8;
-      int blasTop = 0;
-      blasStack[0] = blasRoot;
-      while (blasTop >= 0) {
-        int32_t node = blasStack[blasTop--];
-        int32_t i = node + blasBase;
-        int32_t p, left, right;
-        float d0 = 0.0f, d1 = 0.0f;
-        if (kGpuLayout && layout == 2u) {
-          // BVH_GPU node (intersect.wgsl.ts:453-497): both child boxes inline.
-          float4 g0 = ld4(bvh + i), g1 = ld4(bvh + i + 1), g2 = ld4(bvh + i + 2), g3 = ld4(bvh + i + 3);
-          int32_t count = int32_t(asu(g2.w));
-          p = count > 0 ? -count : 0;
-          left = blasOffset + int32_t(asu(g0.w) * 4u);
-          right = blasOffset + int32_t(asu(g1.w) * 4u);
-          if (p >= 0) {
-            d0 = intersectBox(o, xyz(g0), xyz(g1), linvD, h.tMax);
-            d1 = intersectBox(o, xyz(g2), xyz(g3), linvD, h.tMax);
-          } else {
-            i = blasBase + blasOffset + int32_t(asu(g3.w)) - 2;  // records at i + 2
-          }
-        } else {
-          float4 n1 = ld4(bvh + i);
-          p = asi(n1.w);
-          left = node + 2;
-          right = p + blasOffset;
-          if (p >= 0) {
-            visitInterior(bvh, blasBase, blasOffset, true, o, linvD, h.tMax, left, right, ld4(bvh + left + blasBase),
-                          ld4(bvh + left + 1 + blasBase), ld4(bvh + right + blasBase),
-                          ld4(bvh + right + 1 + blasBase), blasStack, blasTop);
-            continue;
-          }
-        }
-        if (p >= 0) {
-          if (d0 > d1) {
-            if (d0 > 0.0f && blasTop + 1 < MTC_MAX_STACK) blasStack[++blasTop] = left;
-            if (d1 > 0.0f && blasTop + 1 < MTC_MAX_STACK) blasStack[++blasTop] = right;
-          } else {
-            if (d1 > 0.0f && blasTop + 1 < MTC_MAX_STACK) blasStack[++blasTop] = right;
-            if (d0 > 0.0f && blasTop + 1 < MTC_MAX_STACK) blasStack[++blasTop] = left;
-          }
-          continue;
-        }
-        int32_t primitiveCount = -p;
-        int32_t primitiveOffset = i + 2;
-        for (int32_t k = 0; k < primitiveCount; k++) {
-          int32_t triangleIndex = primitiveOffset + k;
-          if (bounces > 0 && triangleIndex == currentTri && insIdx == currentIns) continue;
-          float4 r3 = ld4(bvh + triangleIndex);
-          V3 p0 = vertexPosition(s, asi(r3.x) + vertexOffset);
-          V3 p1 = vertexPosition(s, asi(r3.y) + vertexOffset);
-          V3 p2 = vertexPosition(s, asi(r3.z) + vertexOffset);
-          V3 bary;
-          float t = intersectTriangle(o, p0, p1, p2, maxDim, shear, h.tMax, bary);
-          if (!(t > 0.0f)) continue;
-          V3 candidateNormal = xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0)));
-          if (!doubleSided) {
-            bool matDoubleSided = __ldg(&s.mats[size_t(sideMaterial) * MTC_MATERIAL_VEC4_ROWS + 23].z) > 0.5f;
-            if (!matDoubleSided && xdot(candidateNormal, d) > 0.0f) continue;
-          }
-          h.hitNormal = candidateNormal;
-          h.tMax = t;
-          h.hitBary = bary;
-          if (shadow) {
-            if (kAlpha && !alphaPasses(s, sideMaterial, triangleIndex, asi(r3.x) + vertexOffset,
-                                       asi(r3.y) + vertexOffset, asi(r3.z) + vertexOffset, bary, o + d * t,
-                                       candidateNormal, *alphaSmp)) {
-              h.tMax = tMaxInit;
-              continue;
-            }
-            return true;
-          }
-          h.triangleIndex = triangleIndex;
-          h.insIdx = insIdx;
-        }
-      }
-    }
-  }
-  return false;
-}
-
 // getBVHTraverseCode (intersect.wgsl.ts:213-629) as a restartable state
 // machine, for warps that keep a queue of rays and give a lane a new ray as
 // soon as its current one has finished.  A lane's next piece of work is a

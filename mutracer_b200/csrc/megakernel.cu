@@ -1,11 +1,12 @@
 // sm_100a kernels of the path tracer and their C-ABI entry points:
-//  - k_trace:      plain megakernel, one thread per pixel, all requested
+//  - k_trace:      plain megakernel, one lane per pixel, all requested
 //                  samples of that pixel in order (the progressive pass of
 //                  rayTrace.compute.ts:1157-1263 repeated `samples` times);
 //  - k_batch:      persistent multi-job megakernel; each warp pulls
 //                  (job, 32-pixel tile) work items from one global counter
-//                  and runs every sample of its tile in order, so a job's
-//                  image is bit-identical alone and in a batch;
+//                  for its lanes, which run every sample of their pixel in
+//                  order, so a job's image is bit-identical alone and in a
+//                  batch (mixed jobs: 91 ms, with free-running warps 225);
 //  - k_first_hit:  querySceneSoftware (intersect.wgsl.ts:660-684);
 //  - k_sample_maps: raw material-map lookups (sampleMap) for parity checks;
 //  - k_refit_*:    TLAS refit (bvhAccel.ts:579-740) on the device.
@@ -22,13 +23,6 @@ using namespace mt;
 
 namespace {
 
-// 8x16 pixels per CTA, so a warp covers an 8x4 block (measured 0.5 % faster
-// than 16x2 warps, 1 % faster than 32x1).
-#ifndef MT_TRACE_TILE_W
-#define MT_TRACE_TILE_W 8
-#endif
-constexpr int kTileW = MT_TRACE_TILE_W, kTileH = 128 / MT_TRACE_TILE_W;  // plain kernel CTA tile
-
 __device__ __forceinline__ void flushCounters(const Counters &cnt, uint32_t paths, mtc_counters *out) {
   if (!out) return;
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(&out->kernel_launches, 1ull);
@@ -44,30 +38,67 @@ __device__ __forceinline__ void flushCounters(const Counters &cnt, uint32_t path
   }
 }
 
-// The plain kernel at 16 CTAs of 128 threads per SM (full occupancy, 32
-// registers): it is bound by dependent-load latency, and the warps hide more
-// of it than the spilled state costs (measured 11 % faster than 2 CTAs at
-// 255 registers; 4, 8 and 12 CTAs in between).
-#ifndef MT_TRACE_MIN_BLOCKS
-#define MT_TRACE_MIN_BLOCKS 16
-#endif
+// The pixels of one image, handed out in 8x4 tiles: the grid's blocks take
+// turns at runs of one tile per warp, and a block's lanes claim the pixels of
+// its runs one by one.
+struct ImageClaims {
+  const JobData &J;
+  uint32_t samples;
+  uint32_t *cursor;  // shared: the block's next unit (pixel of a tile)
+  uint32_t run;      // tiles per run
+  bool exhausted = false;
+
+  MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &left) {
+    const uint32_t lane = threadIdx.x & 31u, tilesX = (J.width + 7u) / 8u, tiles = tilesX * ((J.height + 3u) / 4u);
+    unsigned asking = __ballot_sync(0xffffffffu, wants);
+    while (asking && !exhausted) {
+      uint32_t u = 0;
+      if (lane == 0) u = atomicAdd(cursor, uint32_t(__popc(asking)));
+      u = __shfl_sync(0xffffffffu, u, 0) + __popc(asking & ((1u << lane) - 1u));
+      const uint32_t k = u / 32u, in = u % 32u;
+      const uint64_t tile = (uint64_t(k / run) * gridDim.x + blockIdx.x) * run + k % run;
+      if (wants && tile < tiles) {
+        x = uint32_t(tile) % tilesX * 8u + in % 8u;
+        y = uint32_t(tile) / tilesX * 4u + in / 8u;
+        if (x < J.width && y < J.height) {
+          job = &J;
+          left = samples;
+          wants = false;
+        }
+      }
+      // Tiles ascend with the cursor: the last asking lane's tells whether
+      // any is left.
+      exhausted = __any_sync(0xffffffffu, wants && tile >= tiles);
+      asking = __ballot_sync(0xffffffffu, wants);
+    }
+  }
+};
+
+// The plain megakernel.  Bound by instruction fetch and by the latency of its
+// spilled state; with the 32 warps of an SM's block in step 4 samples of the
+// 4M-triangle instanced scene at 960x540 take 29.2 ms (64 free-running warps
+// an SM with one thread per pixel: 67.2), 8 of the Cornell box at 512x512 13.8
+// (29.6), one of the glass scene at 640x360 24.0 (85.2), one of a 256x256
+// Cornell box 1.1 (2.5).  Free-running warps that trace and shade together,
+// or that shade once 8, 12 or 20 lanes wait, are slower than one thread per
+// pixel: it is the fetches shared by the block that pay.
 template <bool kGpuLayout>
-__global__ void __launch_bounds__(kTileW *kTileH, MT_TRACE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kPixelThreads, 1)
     k_trace(const __grid_constant__ JobData J, uint32_t samples, mtc_counters *counters) {
-  uint32_t lx = threadIdx.x % kTileW, ly = threadIdx.x / kTileW;
-  uint32_t x = blockIdx.x * kTileW + lx, y = blockIdx.y * kTileH + ly;
+  __shared__ float columns[kPixelThreads / 32][9 * 32];
+  __shared__ uint32_t cursor;
+  if (threadIdx.x == 0) cursor = 0;
+  __syncthreads();
   Counters cnt;
   uint32_t paths = 0;
-  if (x < J.width && y < J.height) {
-    tracePixelSamples<kGpuLayout>(J, x, y, samples, cnt);
-    paths = samples;
-  }
+  ImageClaims claims{J, samples, &cursor, blockDim.x / 32u};
+  tracePixels<kGpuLayout>(claims, cnt, paths, &columns[threadIdx.x / 32u][threadIdx.x & 31u]);
   flushCounters(cnt, paths, counters);
 }
 
 // Persistent batched kernel over a job table (batch_table.cuh).
 template <bool kGpuLayout>
-__global__ void __launch_bounds__(128, MT_BATCH_MIN_BLOCKS)
+__global__ void __launch_bounds__(kPixelThreads, 1)
     k_batch(const BatchHeader *__restrict__ header, uint32_t *queue, mtc_counters *counters, uint32_t grain,
             uint32_t *status) {
   Counters cnt;
@@ -292,11 +323,17 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
     return MT_ERROR_INVALID_ARGUMENT;
   if (samples == 0) return MT_OK;
   JobData J = makeJob(scene, camera, uniform, out, samples);
-  dim3 grid((J.width + kTileW - 1) / kTileW, (J.height + kTileH - 1) / kTileH);
-  if (scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT)
-    k_trace<true><<<grid, kTileW * kTileH, 0, (cudaStream_t)stream>>>(J, samples, counters);
-  else
-    k_trace<false><<<grid, kTileW * kTileH, 0, (cudaStream_t)stream>>>(J, samples, counters);
+  int device = 0, sms = 148;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  // One block an SM; an image with fewer pixels than that has threads for is
+  // spread over all SMs in smaller blocks.
+  const uint64_t tiles = uint64_t((J.width + 7) / 8) * ((J.height + 3) / 4);
+  const uint64_t perSm = (tiles + uint64_t(sms) - 1) / uint64_t(sms);
+  const uint32_t warps = uint32_t(std::min<uint64_t>(kPixelThreads / 32, std::max<uint64_t>(1, perSm)));
+  const uint32_t grid = uint32_t(std::min<uint64_t>(uint64_t(sms), std::max<uint64_t>(1, (tiles + warps - 1) / warps)));
+  auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_trace<true> : k_trace<false>;
+  kernel<<<grid, warps * 32u, 0, (cudaStream_t)stream>>>(J, samples, counters);
   return cudaStatus(cudaGetLastError());
 }
 
