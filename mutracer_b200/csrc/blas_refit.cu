@@ -9,7 +9,8 @@
 // Math.min/max of its two children's boxes.  Here the cached data is a plan
 // of node offsets grouped by depth, built once on the device by a top-down
 // walk (mtc_blas_refit_prepare); a refit then runs one kernel per depth,
-// deepest first, so every child box is final before its parent reads it.
+// deepest first, so every child box is final before its parent reads it, and
+// one block for the depths near the root.
 // Min/max are exact and order independent (-0 below +0), so the boxes equal
 // the reference's bit for bit.  The reference also sums the nodes' surface
 // areas for its rebuild hint; the device sums the same per-node terms in a
@@ -107,11 +108,14 @@ __global__ void k_plan_close_level(Plan p, uint32_t level) {
 }
 
 // One depth of refitBLAS (bvhAccel.ts:832-868): leaves from their vertices,
-// interior nodes from their (already refitted) children.
-__global__ void __launch_bounds__(kThreads) k_refit_blas_level(Plan p, float4 *bvh, uint32_t level,
-                                                               const float *pos, uint32_t vertexCount) {
+// interior nodes from their (already refitted) children; thread `first` of
+// `threads`.  Bound by random child and vertex gathers.  (One launch in which
+// the second child to finish goes on with its parent took 0.53 ms for 2M
+// triangles: a device-wide fence per node costs more than the launches.)
+__device__ __forceinline__ void refitLevel(const Plan &p, float4 *bvh, uint32_t level, const float *pos,
+                                           uint32_t vertexCount, uint32_t first, uint32_t threads) {
   const uint32_t begin = p.levelStart[level], end = p.levelStart[level + 1];
-  for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = begin + first; i < end; i += threads) {
     const uint32_t o = p.nodes[i];
     float4 a = bvh[o], b = bvh[o + 1];
     const int32_t w = __float_as_int(a.w);
@@ -142,20 +146,42 @@ __global__ void __launch_bounds__(kThreads) k_refit_blas_level(Plan p, float4 *b
   }
 }
 
-// Deterministic sum of the per-node terms (fixed strided order, then a fixed
-// tree), one CTA.
-__global__ void __launch_bounds__(1024) k_area_sum(Plan p, double *out) {
-  __shared__ double part[1024];
-  const uint32_t n = p.h->nodeCount < p.h->capacity ? p.h->nodeCount : p.h->capacity;
+__global__ void __launch_bounds__(kThreads) k_refit_blas_level(Plan p, float4 *bvh, uint32_t level,
+                                                               const float *pos, uint32_t vertexCount) {
+  refitLevel(p, bvh, level, pos, vertexCount, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// Depths `levels` - 1 to 0 in one block: depth d has 2^d nodes at most, so
+// kTopLevels of them are a launch instead of as many small ones.
+constexpr uint32_t kTopLevels = 11;
+__global__ void __launch_bounds__(1024) k_refit_blas_top(Plan p, float4 *bvh, uint32_t levels, const float *pos,
+                                                         uint32_t vertexCount) {
+  for (uint32_t level = levels; level-- > 0;) {
+    refitLevel(p, bvh, level, pos, vertexCount, threadIdx.x, 1024u);
+    __syncthreads();
+  }
+}
+
+// Deterministic sum of the per-node terms, in two launches of the same kernel:
+// every block sums a run of terms (fixed strided order, then a fixed tree) and
+// keeps the result in place of the run's first term; then one block sums those.
+// (One block alone took 0.14 ms for the 2M terms of 2M triangles.)
+constexpr uint32_t kAreaBlocks = 296;
+__global__ void __launch_bounds__(kThreads) k_area_sum(Plan p, bool last, double *out) {
+  __shared__ double part[kThreads];
+  const uint32_t n = min(p.h->nodeCount, p.h->capacity), run = (n + kAreaBlocks - 1u) / kAreaBlocks;
+  const uint32_t step = last ? run : 1u, begin = last ? 0u : blockIdx.x * run;
+  const uint32_t end = last ? n : min(n, begin + run);
   double s = 0.0;
-  for (uint32_t i = threadIdx.x; i < n; i += 1024) s = __dadd_rn(s, p.area[i]);
+  for (uint64_t i = begin + uint64_t(threadIdx.x) * step; i < end; i += uint64_t(kThreads) * step)
+    s = __dadd_rn(s, p.area[i]);
   part[threadIdx.x] = s;
   __syncthreads();
-  for (int w = 512; w; w >>= 1) {
+  for (int w = kThreads / 2; w; w >>= 1) {
     if (threadIdx.x < w) part[threadIdx.x] = __dadd_rn(part[threadIdx.x], part[threadIdx.x + w]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = part[0];
+  if (threadIdx.x == 0 && (last || begin < end)) *(last ? out : p.area + begin) = part[0];
 }
 
 mt_status cudaStatus(cudaError_t e) {
@@ -167,7 +193,7 @@ mt_status cudaStatus(cudaError_t e) {
 int gridFor(uint32_t) {
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  return sms * 4;
+  return sms * 8;
 }
 
 }  // namespace
@@ -221,9 +247,14 @@ mt_status mtc_refit_blas(void *bvh, uint64_t bvh_vec4_count, const void *plan, u
   planBytes(bvh_vec4_count, &p, static_cast<char *>(const_cast<void *>(plan)));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = gridFor(0);
-  for (uint32_t level = levels; level-- > 0;)
+  const uint32_t top = levels < kTopLevels ? levels : kTopLevels;
+  for (uint32_t level = levels; level-- > top;)
     k_refit_blas_level<<<grid, kThreads, 0, st>>>(p, static_cast<float4 *>(bvh), level, positions, vertex_count);
-  if (surface_area) k_area_sum<<<1, 1024, 0, st>>>(p, surface_area);
+  k_refit_blas_top<<<1, 1024, 0, st>>>(p, static_cast<float4 *>(bvh), top, positions, vertex_count);
+  if (surface_area) {
+    k_area_sum<<<kAreaBlocks, kThreads, 0, st>>>(p, false, nullptr);
+    k_area_sum<<<1, kThreads, 0, st>>>(p, true, surface_area);
+  }
   return cudaStatus(cudaGetLastError());
 }
 
