@@ -41,7 +41,11 @@
 
 namespace {
 
-constexpr uint32_t kSmallLimit = 256;   // subtree roots this small are finished by one warp
+// Subtree roots this small are finished by one warp.  256 left an SM 12 warps'
+// worth of shared memory and twice the serial chain per warp: 1.19M triangles
+// 5.46 ms, 20,000 triangles 1.74 ms; 128: 4.94 and 1.47 ms; 64: 5.13 and 1.38
+// (one more level over the whole chip); 512: 7.07 and 2.14.
+constexpr uint32_t kSmallLimit = 128;
 constexpr uint32_t kChunk = 2048;       // primitives per CTA in the level-synchronous phase
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
