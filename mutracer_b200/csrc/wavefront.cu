@@ -7,12 +7,13 @@
 // event loop (rayTrace.compute.ts:891-946) is cut at its traversals into
 // separate kernels that each see a queue of path slots:
 //
-//   k_wf_extend  closest hit of every queued extension ray (traverse<false>)
+//   k_wf_extend  closest hit of every queued extension ray
 //   k_wf_shade   surface interaction, material, completeVertex, shadeVertex
 //                (shadeStep, the same out-of-line code the megakernel calls);
-//                queues the NEE shadow ray and either the continuation or the
-//                finished sample
-//   k_wf_shadow  the NEE visibility tests (traverse<true>)
+//                queues the NEE shadow ray and either the continuation (of the
+//                path, or of its pixel where nothing is left to wait for) or
+//                the finished sample
+//   k_wf_shadow  the NEE visibility tests
 //   k_wf_finish  accumulation of finished samples (endSample) and the start of
 //                the pixel's next sample or of a new pixel (beginSample)
 //
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
       v.classCursor[k] = 0;
     }
   }
+  uint32_t paths = 0;
   const uint32_t n = v.q->rayCount[cur];
   const uint32_t *queue = regroup ? v.sortedQueue : v.rayQueue[cur];
   __shared__ uint32_t taken;
@@ -498,6 +500,18 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
     bool ended = isSpectral(J)   ? shadeStepSpectral(c, ps, v.spectral[s], h)
                  : alphaSplit(J) ? shadeStepAlpha(c, ps, v.spectral[s], h)
                                  : shadeStep(c, ps, v.spectral[s], h);
+    // Most RGB paths end without a shadow ray to wait for (misses, light and
+    // environment hits): accumulated here, their pixel's next sample started,
+    // while the path sample is at hand.  k_wf_finish had to fetch and rewrite
+    // the slot for them (10.9 -> 1.4 ms a frame for 3 ms more here, 8 samples
+    // of the 1080p instanced scene).
+    if (ended && !c.shadow.valid && sl.left > 0u && !isSpectral(J) && !alphaSplit(J)) {
+      endSample(J, sl.x + sl.y * J.width, ps);
+      paths++;
+      sl.left--;
+      beginSample(c, sl.x, sl.y, ps, v.spectral[s]);
+      ended = false;
+    }
     copyPathSample(sl.ps, ps);
     sl.smp = c.smp;
     sl.shadow = c.shadow;
@@ -505,7 +519,7 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
     if (ended) enqueue(v.finishQueue, &v.q->finishCount, s);
     else enqueueRay(v, cur ^ 1u, s);
   }
-  flush(v, 0, 0, 0);
+  flush(v, 0, 0, paths);
 }
 
 // NEE visibility of the queued shadow rays (intersectSceneShadow).  An
