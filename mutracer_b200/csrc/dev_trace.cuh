@@ -357,7 +357,7 @@ struct TraversalHit {
 // instanced scene (1.45M bounce rays, 2.56 ms).  Repeating node visits while
 // enough lanes need one, the header word kept with each stack entry, paired
 // f32 box tests, and the shear of the watertight test computed at leaves
-// (2.3 a ray) instead of instances entered (11.4): 717 at 15 lanes, 1.9 ms.
+// (2.3 a ray) instead of instances entered (11.4): 733 at 12.4 lanes, 1.98 ms.
 // Paired box tests alone are 6 % of the 1080p instanced render.
 //
 // Dense and sparse queues want different waits.  A warp with many rays behind

@@ -38,41 +38,55 @@ __device__ __forceinline__ void flushCounters(const Counters &cnt, uint32_t path
   }
 }
 
-// The pixels of one image, handed out in 8x4 tiles: the grid's blocks take
-// turns at runs of one tile per warp, and a block's lanes claim the pixels of
-// its runs one by one.
+// The pixels of one image in the order of its 8x4 tiles: the grid's blocks take
+// turns at runs of `run` of them, which a block's lanes claim one by one.  Of
+// each warp `lanes` lanes ask: a small image is spread over all warps an SM
+// holds, a few lanes in each, rather than over full warps of a few.
 struct ImageClaims {
   const JobData &J;
   uint32_t samples;
-  uint32_t *cursor;  // shared: the block's next unit (pixel of a tile)
-  uint32_t run;      // tiles per run
+  uint32_t *cursor;  // shared: the block's next pixel
+  uint32_t run, lanes;
   bool exhausted = false;
 
   MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &left) {
-    const uint32_t lane = threadIdx.x & 31u, tilesX = (J.width + 7u) / 8u, tiles = tilesX * ((J.height + 3u) / 4u);
+    const uint32_t lane = threadIdx.x & 31u, tilesX = (J.width + 7u) / 8u;
+    const uint64_t units = uint64_t(tilesX) * ((J.height + 3u) / 4u) * 32u;
+    wants = wants && lane < lanes;
     unsigned asking = __ballot_sync(0xffffffffu, wants);
     while (asking && !exhausted) {
-      uint32_t u = 0;
-      if (lane == 0) u = atomicAdd(cursor, uint32_t(__popc(asking)));
-      u = __shfl_sync(0xffffffffu, u, 0) + __popc(asking & ((1u << lane) - 1u));
-      const uint32_t k = u / 32u, in = u % 32u;
-      const uint64_t tile = (uint64_t(k / run) * gridDim.x + blockIdx.x) * run + k % run;
-      if (wants && tile < tiles) {
-        x = uint32_t(tile) % tilesX * 8u + in % 8u;
-        y = uint32_t(tile) / tilesX * 4u + in / 8u;
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(cursor, uint32_t(__popc(asking)));
+      k = __shfl_sync(0xffffffffu, k, 0) + __popc(asking & ((1u << lane) - 1u));
+      const uint64_t u = (uint64_t(k / run) * gridDim.x + blockIdx.x) * run + k % run;
+      if (wants && u < units) {
+        const uint32_t tile = uint32_t(u / 32u), in = uint32_t(u % 32u);
+        x = tile % tilesX * 8u + in % 8u;
+        y = tile / tilesX * 4u + in / 8u;
         if (x < J.width && y < J.height) {
           job = &J;
           left = samples;
           wants = false;
         }
       }
-      // Tiles ascend with the cursor: the last asking lane's tells whether
-      // any is left.
-      exhausted = __any_sync(0xffffffffu, wants && tile >= tiles);
+      // Pixels ascend with the cursor: none is left once one lies past the
+      // image.
+      exhausted = __any_sync(0xffffffffu, wants && u >= units);
       asking = __ballot_sync(0xffffffffu, wants);
     }
   }
 };
+
+// Small images: up to 256 pixels an SM go to 8 warps of one block, a few lanes
+// each.  Few lanes mean little divergence: 61x47 pixels of the instanced scene
+// take 4.7 ms that way, 9.3 in full warps, 13.0 with one thread per pixel in
+// free-running blocks; 128x72 of glass 11.0, 17.1 and 17.8.  (16 warps: 5.2 and
+// 12.3, and 5 % slower on a 256x256 Cornell box.)  Where paths hardly diverge
+// the block's meetings cost more than that gives: 61x47 of the Cornell box 1.96
+// against 1.60 ms.  Up to kAlonePixels an SM, each pixel gets a block of one
+// warp: nothing to share, no one to wait for (17x13 pixels x 16 samples of the
+// Cornell box 5.1 ms, in pairs 5.9).
+constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
 
 // The plain megakernel.  Bound by instruction fetch and by the latency of its
 // spilled state; with the 32 warps of an SM's block in step 4 samples of the
@@ -84,14 +98,14 @@ struct ImageClaims {
 // pixel: it is the fetches shared by the block that pay.
 template <bool kGpuLayout>
 __global__ void __launch_bounds__(kPixelThreads, 1)
-    k_trace(const __grid_constant__ JobData J, uint32_t samples, mtc_counters *counters) {
+    k_trace(const __grid_constant__ JobData J, uint32_t samples, uint32_t lanes, mtc_counters *counters) {
   __shared__ float columns[kPixelThreads / 32][9 * 32];
   __shared__ uint32_t cursor;
   if (threadIdx.x == 0) cursor = 0;
   __syncthreads();
   Counters cnt;
   uint32_t paths = 0;
-  ImageClaims claims{J, samples, &cursor, blockDim.x / 32u};
+  ImageClaims claims{J, samples, &cursor, blockDim.x / 32u * lanes, lanes};
   tracePixels<kGpuLayout>(claims, cnt, paths, &columns[threadIdx.x / 32u][threadIdx.x & 31u]);
   flushCounters(cnt, paths, counters);
 }
@@ -167,17 +181,21 @@ struct FirstHitSource {
 };
 
 constexpr int kHitThreads = 128;
+// Up to this many vec4 (the 47 of the Cornell box; the smallest mesh scenes have
+// thousands) a BVH counts as small: 832,000 rays 260 us in step, 324 us with
+// lanes taking rays as they finish, 249 us with one ray a thread.
+constexpr uint64_t kUniformNodes = 1024;
 template <bool kGpuLayout>
 __global__ void __launch_bounds__(kHitThreads, 5)
     k_first_hit(const __grid_constant__ DevScene s, int32_t blasBase, int32_t isEmpty, const float4 *rays,
-                uint32_t count, uint32_t raysPerWarp, mtc_hit *hits) {
+                uint32_t count, uint32_t raysPerWarp, uint32_t refillLanes, mtc_hit *hits) {
   __shared__ WarpRays warpRays[kHitThreads / 32];
   const uint64_t first = (uint64_t(blockIdx.x) * (kHitThreads / 32) + threadIdx.x / 32u) * raysPerWarp;
   if (first >= count) return;
   const uint32_t end = uint32_t(min(uint64_t(count), first + raysPerWarp));
   FirstHitSource src{s, rays, hits, blasBase, isEmpty != 0, uint32_t(first)};
   traceQueue<false, kGpuLayout, false>(src, end, min(32u, raysPerWarp), raysPerWarp >= kDenseRays ? kNodeLanes : 1u,
-                                       4u, 8u, warpRays[threadIdx.x / 32u]);
+                                       refillLanes, 8u, warpRays[threadIdx.x / 32u]);
 }
 
 // read_average (native/host/src/lib.rs:343-364): each f32 of an accumulation
@@ -326,14 +344,19 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
   int device = 0, sms = 148;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  // One block an SM; an image with fewer pixels than that has threads for is
-  // spread over all SMs in smaller blocks.
-  const uint64_t tiles = uint64_t((J.width + 7) / 8) * ((J.height + 3) / 4);
-  const uint64_t perSm = (tiles + uint64_t(sms) - 1) / uint64_t(sms);
-  const uint32_t warps = uint32_t(std::min<uint64_t>(kPixelThreads / 32, std::max<uint64_t>(1, perSm)));
-  const uint32_t grid = uint32_t(std::min<uint64_t>(uint64_t(sms), std::max<uint64_t>(1, (tiles + warps - 1) / warps)));
+  // One block an SM, of as many warps as it has pixels for.
+  const uint64_t units = uint64_t((J.width + 7) / 8) * ((J.height + 3) / 4) * 32u;
+  const uint64_t perSm = std::max<uint64_t>(1, (units + uint64_t(sms) - 1) / uint64_t(sms));
+  uint32_t warps = uint32_t(std::min<uint64_t>(
+      kPixelThreads / 32, perSm <= kSpreadWarps * 32u ? std::min<uint64_t>(kSpreadWarps, perSm) : (perSm + 31) / 32));
+  uint32_t lanes = uint32_t(std::min<uint64_t>(32, (perSm + warps - 1) / warps));
+  uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms), units)));
+  if (perSm <= kAlonePixels) {
+    warps = lanes = 1;
+    grid = uint32_t(std::max<uint64_t>(1, units));
+  }
   auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_trace<true> : k_trace<false>;
-  kernel<<<grid, warps * 32u, 0, (cudaStream_t)stream>>>(J, samples, counters);
+  kernel<<<grid, warps * 32u, 0, (cudaStream_t)stream>>>(J, samples, lanes, counters);
   return cudaStatus(cudaGetLastError());
 }
 
@@ -346,14 +369,17 @@ mt_status mtc_query_first_hit(const mtc_scene_view *scene, const float *rays, ui
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   // A few rays: one a warp, which then waits for no other.  Many: up to 256 a
   // warp, as long as there are enough warps left to fill the SMs three times.
-  const uint64_t warps = uint64_t(sms) * 5u * (kHitThreads / 32) * 3u;
-  const uint32_t perWarp = uint32_t(std::min<uint64_t>(256u, (count + warps - 1u) / warps));
+  // In a small BVH rays take much the same steps: 32 a warp that start and
+  // finish together, once there is a warp of them for every scheduler.
+  const bool together = scene->bvh_vec4_count <= kUniformNodes;
+  const uint64_t warps = uint64_t(sms) * (together ? 4u : 5u * (kHitThreads / 32) * 3u);
+  const uint32_t perWarp = uint32_t(std::min<uint64_t>(together ? 32u : 256u, (count + warps - 1u) / warps));
   const uint32_t perBlock = perWarp * (kHitThreads / 32);
   const uint32_t grid = uint32_t((uint64_t(count) + perBlock - 1u) / perBlock);
   const int32_t blasBase = scene->blas_offset;
   auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_first_hit<true> : k_first_hit<false>;
   kernel<<<grid, kHitThreads, 0, (cudaStream_t)stream>>>(toDev(scene), blasBase, scene->instance_count == 0,
-                                                         (const float4 *)rays, count, perWarp, hits);
+                                                         (const float4 *)rays, count, perWarp, together ? 32u : 4u, hits);
   return cudaStatus(cudaGetLastError());
 }
 

@@ -447,8 +447,9 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_regroup(StreamView v) {
 // and over the code fetched it apart (28 of 55 stall cycles per issue waited
 // for instructions).  So the class-ordered queue is handed out in chunks from
 // one counter, which keeps the SM's blocks in one class at a time, and the
-// four warps of a block start each chunk together (3 of 16 stall cycles, 2.61
-// -> 1.89 ms for 1.45M rays).  With fetches shared, more registers and fewer
+// four warps of a block start each chunk together (10.5 of 26 stall cycles; one
+// block of 512 threads an SM in step: 3 of 16, 2.61 -> 1.89 ms for 1.45M rays).
+// With fetches shared, more registers and fewer
 // warps win: 4 blocks at 128 registers against 8 at 64 (124.3 and 125.3 ms,
 // 8 samples of the 1080p instanced scene; 30.9 and 32.8 ms, 16 samples of the
 // Cornell box).  Blocks of 256 and 512 threads: 2 % faster on the first, 2 to
