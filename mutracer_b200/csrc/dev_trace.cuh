@@ -182,11 +182,6 @@ MTD int maxDimension(V3 v) {
   if (v.x > v.y) return v.x > v.z ? 0 : 2;
   return v.y > v.z ? 1 : 2;
 }
-MTD V3 getShear(V3 d, int maxDim) {
-  if (maxDim == 0) return {xd(-d.y, d.x), xd(-d.z, d.x), __frcp_rn(d.x)};
-  if (maxDim == 1) return {xd(-d.z, d.y), xd(-d.x, d.y), __frcp_rn(d.y)};
-  return {xd(-d.x, d.z), xd(-d.y, d.z), __frcp_rn(d.z)};
-}
 // intersect.wgsl.ts:1430-1493; returns t (0 for a miss) and barycentrics.
 MTD float intersectTriangle(V3 o, V3 p0, V3 p1, V3 p2, int maxDim, V3 shear, float tMax, V3 &bary) {
   V3 a = xsub3(p0, o), b = xsub3(p1, o), c = xsub3(p2, o);
@@ -388,8 +383,9 @@ MTD V3 hitNormal(const DevScene &s, int32_t triangleIndex, int32_t insIdx) {
   return xnormalize(xcross(xsub3(p1, p0), xsub3(p2, p0)));
 }
 
-// The values of getShear(d, maxDim), the axes selected before the divisions
-// so that lanes of different dominant axes divide together.
+// The shear of the watertight test (intersect.wgsl.ts:1500-1521), the axes
+// selected before the divisions so that lanes of different dominant axes divide
+// together.
 MTD V3 selectShear(V3 d, int maxDim) {
   const float z = maxDim == 0 ? d.x : maxDim == 1 ? d.y : d.z;
   const float x = maxDim == 0 ? d.y : maxDim == 1 ? d.z : d.x;
