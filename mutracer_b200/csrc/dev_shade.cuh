@@ -4,6 +4,8 @@
 // sampleLight.wgsl.ts, envMap.wgsl.ts, background.wgsl.ts and
 // materialBuffer.wgsl.ts (paths relative to src/renderer/wgsl/).
 #pragma once
+#include <type_traits>
+
 #include "dev_bsdf.cuh"
 #include "dev_trace.cuh"
 #include "spectrum_cdf.h"
@@ -850,14 +852,21 @@ struct ShadowQuery {
   bool valid;
 };
 
+// What shading needs of a lane's job besides its path.
 struct Ctx {
-  const JobData &J;
+  const JobData *job;
   Sampler smp;
   BsdfContext bc;
-  Counters cnt;
   ShadowQuery shadow;
-  MTD uint32_t candidateCount() const { return uint32_t(max(J.u.direct_light_candidates, 1)); }
+  MTD uint32_t candidateCount() const { return uint32_t(max(job->u.direct_light_candidates, 1)); }
 };
+// A lane of the megakernels takes on one job after another.
+static_assert(std::is_copy_assignable<Ctx>::value, "Ctx is assigned at every claim");
+MTD Ctx startContext(const JobData &J) {
+  return Ctx{&J, Sampler(),
+             BsdfContext{J.s.lut, (J.s.flags & MTC_SCENE_HAS_MEDIUM) != 0u, feature(J, MTC_FEATURE_HAS_THIN_FILM)},
+             ShadowQuery()};
+}
 
 // rayTrace.compute.ts:264-284
 MTD float neeMISWeight(const Ctx &c, float lightPdf, float scatteringPdf) {
@@ -937,14 +946,14 @@ MTD bool finishDirectLight(Ctx &c, const SurfaceInteraction &si, Path &path, V3 
     visDir = normalize(to);
   }
   if (isSurface && cosThetaL < 0.0f && ls.sourceType == 0u) {
-    float4 bg = sampleSceneBackground(c.J, visDir);
+    float4 bg = sampleSceneBackground(*c.job, visDir);
     Li = V3{bg.x, bg.y, bg.z} * bg.w;
   }
   // Spectral scenes use channel-independent RIS (WGPURayTracePass.ts:1349,
   // sampleMaterial.wgsl.ts:119-140): with three wavelengths the radiance is
   // filtered after the target, and each RGB component weighs 1/3.
-  const bool spectral = isSpectral(c.J);
-  const bool threeWavelengths = spectral && c.J.u.dispersion_wavelengths != 1;
+  const bool spectral = isSpectral(*c.job);
+  const bool threeWavelengths = spectral && c.job->u.dispersion_wavelengths != 1;
   if (spectral && !threeWavelengths) Li = spectralFilter(Li, si.spectralChannel);
   float mis = ls.isDelta ? 1.0f : neeMISWeight(c, lightPdf, scatteringPdf);
   if (mis > 0.0f) {
@@ -1025,7 +1034,7 @@ MTD Scattering sampleScattering(Ctx &c, SurfaceInteraction &si, const Material &
       V2 lr = c.smp.s2(c.smp.lightDim(event, 1u));
       float lz = c.smp.s1(c.smp.lightDim(event, 0u));
       V3 rnd = {lr.x, lr.y, (lz + float(min(event, count - 1u))) / float(max(count, 1u))};
-      sampleLightChoiceTable(c.J, si.position, rnd, ls);
+      sampleLightChoiceTable(*c.job, si.position, rnd, ls);
       lightDir = ls.direction;
       if (ls.pdf <= 0.0f || ls.selectionPmf <= 0.0f || maxc(ls.emission) <= 0.0f) continue;
       float cosThetaL = dot(ffnormal, lightDir);
@@ -1061,17 +1070,17 @@ MTD float emissiveHitMisWeight(Ctx &c, const SurfaceInteraction &si, const Path 
                                float doubleSided) {
   float cosLight = dot(si.faceNormal, -path.ray.d);
   if (cosLight <= 0.0f && doubleSided < 0.5f) return 0.0f;
-  if (path.fromEye || c.J.u.light_weight_total <= 0.0f || int(row0.w) == 2) return 1.0f;
+  if (path.fromEye || c.job->u.light_weight_total <= 0.0f || int(row0.w) == 2) return 1.0f;
   float lum = dot(xyz(row3), kLuminance());
   if (lum <= 0.0f || cosLight <= 0.0f) return 1.0f;
   float hd = distance(si.position, path.ray.o);
-  float lightPdf = lum / c.J.u.light_weight_total * hd * hd / fmaxf(cosLight, 1e-8f);
+  float lightPdf = lum / c.job->u.light_weight_total * hd * hd / fmaxf(cosLight, 1e-8f);
   return bsdfMISWeight(c, path.scatteringPdf, lightPdf);
 }
 
 // sampleMaterial.wgsl.ts:316-508
 MTD void sampleMaterial(Ctx &c, SurfaceInteraction &si, Material &ma, Path &path) {
-  const bool hasMedium = (c.J.s.flags & MTC_SCENE_HAS_MEDIUM) != 0u;
+  const bool hasMedium = (c.job->s.flags & MTC_SCENE_HAS_MEDIUM) != 0u;
   float ndv1 = -dot(si.faceNormal, path.ray.d);
   float ndv2 = -dot(si.normal, path.ray.d);
   if ((ma.transmissionWeight > 0.0f || ma.subsurfaceWeight > 0.0f) && ma.thinWalled) {
@@ -1114,11 +1123,11 @@ MTD void sampleMaterial(Ctx &c, SurfaceInteraction &si, Material &ma, Path &path
     }
   }
   if (!mediumSampled) {
-    int mi = uint32_t(si.materialIndex) < c.J.s.matCount ? si.materialIndex : 0;
-    const float4 *md = c.J.s.mats + size_t(mi) * MTC_MATERIAL_VEC4_ROWS;
+    int mi = uint32_t(si.materialIndex) < c.job->s.matCount ? si.materialIndex : 0;
+    const float4 *md = c.job->s.mats + size_t(mi) * MTC_MATERIAL_VEC4_ROWS;
     V3 se = ma.emission;
     if (se.x != 0.0f || se.y != 0.0f || se.z != 0.0f) {
-      if (isSpectral(c.J)) se = spectralFilter(se, si.spectralChannel);
+      if (isSpectral(*c.job)) se = spectralFilter(se, si.spectralChannel);
       float w = emissiveHitMisWeight(c, si, path, ld4(md), ld4(md + 3), ld4(md + 23).z);
       path.li += se * w * path.beta;
     }
@@ -1174,10 +1183,10 @@ MTD void shadeVertex(Ctx &c, V2 uv, Path &path, int &depth, SurfaceInteraction &
   sampleIgnored = false;
   c.smp.bounce = uint32_t(max(depth, 0));
   int matType = ma.materialType;
-  const mtc_trace_uniform &u = c.J.u;
+  const mtc_trace_uniform &u = c.job->u;
   if (!si.hit) {
-    float4 bg = sampleSceneBackground(c.J, path.ray.d);
-    if (isSpectral(c.J)) {
+    float4 bg = sampleSceneBackground(*c.job, path.ray.d);
+    if (isSpectral(*c.job)) {
       V3 f = spectralFilter({bg.x, bg.y, bg.z}, si.spectralChannel);
       bg = make_float4(f.x, f.y, f.z, bg.w);
     }
@@ -1186,12 +1195,12 @@ MTD void shadeVertex(Ctx &c, V2 uv, Path &path, int &depth, SurfaceInteraction &
       path.alpha = bg.w;
       aux.isBlank = bg.w < 0.001f || ((u.background_flags & MTC_BACKGROUND_COLOR) && !(u.background_flags & MTC_BACKGROUND_MAP));
     } else {
-      Ray cam = initCameraRay(c.J, uv);
+      Ray cam = initCameraRay(*c.job, uv);
       bool towardsCam = dot(cam.d, path.ray.d) > 0.0f;
       if (u.transmissive_output_alpha_min < 1.0f) {
         if (towardsCam) path.alpha = fmaxf(path.alpha, bg.w); else path.alpha = 1.0f;
       }
-      if (!useEnvmap(c.J) && towardsCam)
+      if (!useEnvmap(*c.job) && towardsCam)
         path.li += path.beta * bsdfMISWeight(c, path.scatteringPdf, 1.0f) * V3{bg.x, bg.y, bg.z};
     }
     path.abort = true;
@@ -1213,7 +1222,7 @@ MTD void shadeVertex(Ctx &c, V2 uv, Path &path, int &depth, SurfaceInteraction &
     if (matType == 0 || matType == 2) {
       if (!(ma.transmissionWeight > 0.5f || (ma.specularRoughness <= 0.02f && ma.baseMetalness > 0.98f))) {
         aux.albedo = ma.baseColor;
-        aux.normal = dot(si.normal, si.position - cameraEye(c.J)) > 0.0f ? -si.normal : si.normal;
+        aux.normal = dot(si.normal, si.position - cameraEye(*c.job)) > 0.0f ? -si.normal : si.normal;
         si.albedoSampled = true;
       }
       if (depth > 4) si.albedoSampled = true;
@@ -1228,13 +1237,13 @@ MTD void shadeVertex(Ctx &c, V2 uv, Path &path, int &depth, SurfaceInteraction &
 
 // rayTrace.compute.ts:514-589 completeVertex
 MTD void completeVertex(Ctx &c, Path &path, int &depth, SurfaceInteraction &si, Material &ma, bool sampleIgnored) {
-  const bool spectral = isSpectral(c.J);
+  const bool spectral = isSpectral(*c.job);
   if (spectral && ma.transmissionWeight > 0.001f)
     ma.specularIor = cauchyIor(si.wavelength, ma.specularIor, ma.transmissionDispersionScale, ma.dispersionAbbeNumber);
   if (sampleIgnored) return;
   bool isAlphaOccluded = ma.alpha >= 1.0f ? (c.smp.hashed += 1u, true) : c.smp.hashedSample(3u) < ma.alpha;
-  for (int i = 0; i < c.J.u.lights_count; i++) {
-    Light L = loadLight(c.J, i);
+  for (int i = 0; i < c.job->u.lights_count; i++) {
+    Light L = loadLight(*c.job, i);
     LightSample ls = zeroLightSample();
     float d = intersectLight(path.ray, L, ls);
     ls.pdf *= L.selectionPmf;
@@ -1247,23 +1256,23 @@ MTD void completeVertex(Ctx &c, Path &path, int &depth, SurfaceInteraction &si, 
       path.abort = true;
     }
   }
-  if (useEnvmap(c.J) && !(si.hit && isAlphaOccluded)) {
+  if (useEnvmap(*c.job) && !(si.hit && isAlphaOccluded)) {
     if (path.isNextRefraction) {
-      float4 bg = sampleSceneBackground(c.J, path.ray.d);
+      float4 bg = sampleSceneBackground(*c.job, path.ray.d);
       V3 rgb = {bg.x, bg.y, bg.z};
       if (spectral) rgb = spectralFilter(rgb, si.spectralChannel);
       float w = path.scatteringIsDelta ? 1.0f
-                : bsdfMISWeight(c, path.scatteringPdf, envMapPdf(c.J, environmentUv(c.J, path.ray.d)) * c.J.u.env_light_pmf);
+                : bsdfMISWeight(c, path.scatteringPdf, envMapPdf(*c.job, environmentUv(*c.job, path.ray.d)) * c.job->u.env_light_pmf);
       path.li += path.beta * rgb * (w * bg.w);
       path.alpha = fmaxf(path.alpha, bg.w);
       path.abort = true;
       return;
     }
-    V2 euv = environmentUv(c.J, path.ray.d);
-    V3 emission = xyz(textureLinear(c.J.s.env, c.J.s.envW, c.J.s.envH, euv));
-    float mis = bsdfMISWeight(c, path.scatteringPdf, envMapPdf(c.J, euv) * c.J.u.env_light_pmf);
+    V2 euv = environmentUv(*c.job, path.ray.d);
+    V3 emission = xyz(textureLinear(c.job->s.env, c.job->s.envW, c.job->s.envH, euv));
+    float mis = bsdfMISWeight(c, path.scatteringPdf, envMapPdf(*c.job, euv) * c.job->u.env_light_pmf);
     if (spectral) emission = spectralFilter(emission, si.spectralChannel);
-    if (!(c.J.u.background_flags & MTC_BACKGROUND_COLOR)) path.alpha = 1.0f;
+    if (!(c.job->u.background_flags & MTC_BACKGROUND_COLOR)) path.alpha = 1.0f;
     path.li += path.beta * emission * mis;
     path.abort = true;
   }
@@ -1340,7 +1349,7 @@ MTD bool alphaSplit(const JobData &J) { return (J.s.flags & MTC_SCENE_HAS_ALPHA)
 // ray and thin lens, then integrator() locals (:891-905).  Out of line, like
 // shadeStep and endSample, so every kernel runs one compiled copy.
 static __device__ __noinline__ void beginSample(Ctx &c, uint32_t x, uint32_t y, PathSample &ps, SpectralState &sp) {
-  const JobData &J = c.J;
+  const JobData &J = *c.job;
   const mtc_trace_uniform &u = J.u;
   uint32_t W = J.width;
   uint32_t idx = x + y * W;
@@ -1441,20 +1450,20 @@ MTD bool reusesPrimary(const JobData &J, const PathSample &ps, bool primaryReady
 static __device__ __noinline__ bool shadeStep(Ctx &c, PathSample &ps, SpectralState &sp, const TraversalHit &h) {
   Path &path = ps.path;
   SurfaceInteraction &si = ps.si;
-  const int bounceLimit = max(c.J.u.bounces, 0);
+  const int bounceLimit = max(c.job->u.bounces, 0);
   const int eventLimit = min(bounceLimit * 3, 20);
   const int event = ps.event;
   si.hit = false;
   if (h.insIdx >= 0) {
     si.triangleIndex = h.triangleIndex;
-    completeSurfaceInteraction(c.J, si, sp.tex, h, path.ray.o, path.ray.d);
+    completeSurfaceInteraction(*c.job, si, sp.tex, h, path.ray.o, path.ray.d);
   }
   Material ma;
-  getMaterial(c.J, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
+  getMaterial(*c.job, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
   if (event == 0) {
     if (si.hit && (ma.materialType == 0 || ma.materialType == 2)) {
       ps.aux.albedo = ma.transmissionWeight > 0.5f ? v3(1.0f) : ma.baseColor;
-      ps.aux.normal = dot(si.normal, si.position - cameraEye(c.J)) > 0.0f ? -si.normal : si.normal;
+      ps.aux.normal = dot(si.normal, si.position - cameraEye(*c.job)) > 0.0f ? -si.normal : si.normal;
       si.albedoSampled = ma.transmissionWeight > 0.5f;
     }
     ps.isNotTransparent = ma.transmissionWeight < 0.001f && ma.subsurfaceWeight < 0.001f && ma.alpha > 0.99f;
@@ -1479,7 +1488,7 @@ static __device__ __noinline__ bool shadeStep(Ctx &c, PathSample &ps, SpectralSt
 static __device__ __noinline__ bool shadeStepAlpha(Ctx &c, PathSample &ps, SpectralState &sp, const TraversalHit &h) {
   Path &path = ps.path;
   SurfaceInteraction &si = ps.si;
-  const int bounceLimit = max(c.J.u.bounces, 0);
+  const int bounceLimit = max(c.job->u.bounces, 0);
   const int eventLimit = min(bounceLimit * 3, 20);
   const int event = ps.event;
   Material ma;
@@ -1487,20 +1496,20 @@ static __device__ __noinline__ bool shadeStepAlpha(Ctx &c, PathSample &ps, Spect
     sp.frontPending = false;
     si = sp.primarySi;
     sp.tex = sp.primaryTex;
-    getMaterial(c.J, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
+    getMaterial(*c.job, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
     ma.alpha = 1.0f;
   } else {
     si.hit = false;
     if (h.insIdx >= 0) {
       si.triangleIndex = h.triangleIndex;
-      completeSurfaceInteraction(c.J, si, sp.tex, h, path.ray.o, path.ray.d);
+      completeSurfaceInteraction(*c.job, si, sp.tex, h, path.ray.o, path.ray.d);
     }
-    getMaterial(c.J, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
+    getMaterial(*c.job, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
   }
   if (!sp.primaryReady) {
     if (si.hit && (ma.materialType == 0 || ma.materialType == 2)) {
       ps.aux.albedo = ma.transmissionWeight > 0.5f ? v3(1.0f) : ma.baseColor;
-      ps.aux.normal = dot(si.normal, si.position - cameraEye(c.J)) > 0.0f ? -si.normal : si.normal;
+      ps.aux.normal = dot(si.normal, si.position - cameraEye(*c.job)) > 0.0f ? -si.normal : si.normal;
       si.albedoSampled = ma.transmissionWeight > 0.5f;
     }
     sp.primarySi = si;
@@ -1517,7 +1526,7 @@ static __device__ __noinline__ bool shadeStepAlpha(Ctx &c, PathSample &ps, Spect
   } else if (event == 0 && !sp.front && sp.split) {
     if (si.hit && ma.materialType == 0) {
       ps.aux.albedo = ma.transmissionWeight > 0.5f ? v3(1.0f) : ma.baseColor;
-      ps.aux.normal = dot(si.normal, si.position - cameraEye(c.J)) > 0.0f ? -si.normal : si.normal;
+      ps.aux.normal = dot(si.normal, si.position - cameraEye(*c.job)) > 0.0f ? -si.normal : si.normal;
       si.albedoSampled = ma.transmissionWeight > 0.5f;
     }
   }
@@ -1589,12 +1598,12 @@ static __device__ __noinline__ bool shadeStepSpectral(Ctx &c, PathSample &ps, Sp
                                                       const TraversalHit &h) {
   Path &path = ps.path;
   SurfaceInteraction &si = ps.si;
-  const mtc_trace_uniform &u = c.J.u;
+  const mtc_trace_uniform &u = c.job->u;
   const int bounceLimit = max(u.bounces, 0);
   const int eventLimit = min(bounceLimit * 3, 20);
   int event = ps.event;
   const bool singleWavelength = u.dispersion_wavelengths == 1;
-  const bool spEnabled = !singleWavelength && !(c.J.s.flags & MTC_SCENE_SPECTRAL_INDEPENDENT);
+  const bool spEnabled = !singleWavelength && !(c.job->s.flags & MTC_SCENE_SPECTRAL_INDEPENDENT);
   auto spFork = [&]() {  // spectralPrefix.wgsl.ts:32-36
     sp.spActive = false;
     path.li = spectralFilter(path.li, sp.spChannel);
@@ -1602,23 +1611,23 @@ static __device__ __noinline__ bool shadeStepSpectral(Ctx &c, PathSample &ps, Sp
     si.wavelength = sp.spWavelength;
   };
   Material ma;
-  if (!reusesPrimary(c.J, ps, sp.primaryReady)) {
+  if (!reusesPrimary(*c.job, ps, sp.primaryReady)) {
     si.hit = false;
     if (h.insIdx >= 0) {
       si.triangleIndex = h.triangleIndex;
-      completeSurfaceInteraction(c.J, si, sp.tex, h, path.ray.o, path.ray.d);
+      completeSurfaceInteraction(*c.job, si, sp.tex, h, path.ray.o, path.ray.d);
     }
-    getMaterial(c.J, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
+    getMaterial(*c.job, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
   } else {
     // The primary material is a pure function of the primary vertex.
-    getMaterial(c.J, sp.primarySi.materialIndex, sp.primarySi.instanceIndex, sp.primaryTex.uv, sp.primaryTex.uv1,
+    getMaterial(*c.job, sp.primarySi.materialIndex, sp.primarySi.instanceIndex, sp.primaryTex.uv, sp.primaryTex.uv1,
                 sp.primaryTex.vertexColor, ma);
   }
   if (event == 0) {
     if (!sp.primaryReady) {
       if (si.hit && (ma.materialType == 0 || ma.materialType == 2)) {
         sp.primaryAux.albedo = ma.transmissionWeight > 0.5f ? v3(1.0f) : ma.baseColor;
-        sp.primaryAux.normal = dot(si.normal, si.position - cameraEye(c.J)) > 0.0f ? -si.normal : si.normal;
+        sp.primaryAux.normal = dot(si.normal, si.position - cameraEye(*c.job)) > 0.0f ? -si.normal : si.normal;
         si.albedoSampled = ma.transmissionWeight > 0.5f;
       }
       sp.primarySi = si;
@@ -1682,7 +1691,7 @@ static __device__ __noinline__ bool shadeStepSpectral(Ctx &c, PathSample &ps, Sp
       c.smp.s0 = sp.forkS0;
       c.smp.hashed = sp.forkHashed;
       c.smp.bounce = sp.forkBounce;
-      getMaterial(c.J, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
+      getMaterial(*c.job, si.materialIndex, si.instanceIndex, sp.tex.uv, sp.tex.uv1, sp.tex.vertexColor, ma);
       spFork();
     }
   }
@@ -1826,11 +1835,9 @@ static __device__ __noinline__ void endSample(const JobData &J, uint32_t idx, co
 // left).
 template <bool kGpuLayout, class Claims>
 MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths, float *column) {
-  // A job's Ctx is made anew at each claim; it is only used while left > 0.
-  alignas(16) unsigned char room[sizeof(Ctx)];
-  Ctx &c = *reinterpret_cast<Ctx *>(room);
+  Ctx c{nullptr, Sampler(), BsdfContext(), ShadowQuery()};
   const JobData *job = nullptr;
-  PathSample ps;
+  PathSample ps;  // ps and sp hold a path, and c its job, while left > 0
   SpectralState sp;
   uint32_t x = 0, y = 0, left = 0;
   for (;;) {
@@ -1838,10 +1845,7 @@ MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths, float *colu
     claims.next(wants, job, x, y, left);
     if (wants && left) {
       paths += left;
-      new (room) Ctx{*job, Sampler(),
-                     BsdfContext{job->s.lut, (job->s.flags & MTC_SCENE_HAS_MEDIUM) != 0u,
-                                 feature(*job, MTC_FEATURE_HAS_THIN_FILM)},
-                     Counters(), ShadowQuery()};
+      c = startContext(*job);
       beginSample(c, x, y, ps, sp);
     }
     const bool active = left != 0u;
@@ -1861,8 +1865,9 @@ MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths, float *colu
                !(spectral ? reusesPrimary(*job, ps, sp.primaryReady) : split && sp.frontPending);
       if (extend) cnt.ext++;
     }
-    traceWarp<false, kGpuLayout>(job, extend, ps.path.ray, ps.event != 0, ps.depth > 0 ? ps.si.triangleIndex : -1,
-                                 ps.si.instanceIndex, h, column, nullptr);
+    traceWarp<false, kGpuLayout>(job, extend, ps.path.ray, extend && ps.event != 0,
+                                 extend && ps.depth > 0 ? ps.si.triangleIndex : -1,
+                                 extend ? ps.si.instanceIndex : -1, h, column, nullptr);
     __syncthreads();
     if (active) {
       c.shadow.valid = false;

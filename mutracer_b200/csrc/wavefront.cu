@@ -152,10 +152,6 @@ __device__ __forceinline__ void flush(const StreamView &v, uint32_t ext, uint32_
   }
 }
 
-__device__ __forceinline__ BsdfContext bsdfContext(const JobData &J) {
-  return BsdfContext{J.s.lut, (J.s.flags & MTC_SCENE_HAS_MEDIUM) != 0u, feature(J, MTC_FEATURE_HAS_THIN_FILM)};
-}
-
 // Material classes for regrouping the shading queue: 0 = miss, else 1 + a
 // mask of the lobes the hit material switches on (metal, coat, transmission,
 // fuzz/subsurface/thin film, non-default material type), read from the
@@ -236,7 +232,7 @@ __device__ bool claimPixel(const StreamView &v, uint32_t s) {
     sl.x = x;
     sl.y = y;
     sl.left = J.samples - 1u;
-    Ctx c{J, Sampler(), bsdfContext(J), Counters(), ShadowQuery()};
+    Ctx c = startContext(J);
     alignas(16) PathSample ps;
     beginSample(c, x, y, ps, v.spectral[s]);
     copyPathSample(sl.ps, ps);
@@ -485,7 +481,8 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
     if (s >= v.slotCount) continue;
     Slot &sl = v.slots[s];
     const JobData &J = v.jobs[sl.job];
-    Ctx c{J, sl.smp, bsdfContext(J), Counters(), ShadowQuery()};
+    Ctx c = startContext(J);
+    c.smp = sl.smp;
     c.shadow.valid = false;
     alignas(16) PathSample ps;
     copyPathSample(ps, sl.ps);
@@ -606,7 +603,7 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_finish(StreamView v) {
     bool again;
     if (sl.left > 0u) {
       sl.left--;
-      Ctx c{J, Sampler(), bsdfContext(J), Counters(), ShadowQuery()};
+      Ctx c = startContext(J);
       beginSample(c, sl.x, sl.y, ps, v.spectral[s]);
       copyPathSample(sl.ps, ps);
       sl.smp = c.smp;

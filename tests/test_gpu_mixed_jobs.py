@@ -1,0 +1,67 @@
+"""Lanes of one persistent launch that go from job to job of unlike kinds:
+opaque, alpha-covered and dispersive scenes, so that a warp holds lanes with
+and without coverage draws and a lane's job changes under way.  Each image is
+bit-identical to the job's own, and to the wavefront engine's."""
+import ctypes as C
+
+import pytest
+
+from mutracer_b200 import abi, batch, scene
+from tests.test_gpu_alpha import alpha_room, decode
+
+pytestmark = pytest.mark.gpu
+PARTS = ("color", "normal", "albedo", "catcher")
+
+
+def _same(a, b):
+    import torch
+    return all(torch.equal(getattr(a, k), getattr(b, k)) for k in PARTS)
+
+
+@pytest.fixture(scope="module")
+def scenes(cuda):
+    hosts = [decode(alpha_room(41, 23)), scene.SceneHost("cornell", 37, 29, 2),
+             scene.SceneHost("glass_spheres", 19, 11, 4, (4,)), decode(alpha_room(9, 31))]
+    return [scene.DeviceScene(h, cuda) for h in hosts], [3, 4, 1, 2]
+
+
+@pytest.fixture(scope="module")
+def alone(cuda, scenes):
+    import torch
+    jobs = [batch.RenderJob(d, s, device=cuda) for d, s in zip(*scenes)]
+    for j in jobs:
+        j.render_alone()
+    torch.cuda.synchronize()
+    return jobs
+
+
+# One block of one warp an SM hands every lane several jobs; tiles of one
+# pixel's width put unlike jobs side by side in a warp.
+@pytest.mark.parametrize("cfg", [(0, 0, 0, 0), (32, 1, 1, 16), (128, 8, 4, 3)])
+def test_unlike_jobs_share_a_persistent_launch(cuda, scenes, alone, cfg):
+    import torch
+    devs, spp = scenes
+    order = [0, 1, 2, 3, 1, 0]
+    jobs = [batch.RenderJob(devs[k], spp[k], device=cuda) for k in order]
+    b = batch.Batch(len(jobs), abi.BatchConfig.make(*cfg), cuda)
+    b.set_jobs(jobs)
+    b.launch()
+    torch.cuda.synchronize()
+    for k, j in zip(order, jobs):
+        assert _same(alone[k].acc, j.acc), k
+
+
+def test_unlike_jobs_agree_in_the_other_engines(cuda, scenes, alone):
+    import torch
+    devs, spp = scenes
+    jobs = [batch.RenderJob(d, s, device=cuda) for d, s in zip(devs, spp)]
+    sb = batch.StreamBatch(len(jobs), stream_config=abi.StreamConfig.make(slots=1024), device=cuda)
+    sb.set_jobs(jobs)
+    sb.run()
+    fixed = [batch.RenderJob(d, s, device=cuda) for d, s in zip(devs, spp)]
+    descs = (abi.JobDesc * len(fixed))(*[j.desc(j.spp) for j in fixed])
+    abi.check(abi.lib().mtc_trace_batch_noalloc(descs, len(fixed), None, None, None,
+                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    for want, a, b in zip(alone, jobs, fixed):
+        assert _same(want.acc, a.acc) and _same(want.acc, b.acc)
