@@ -1545,8 +1545,11 @@ static __device__ __noinline__ bool shadeStepAlpha(Ctx &c, PathSample &ps, Spect
 // End of an alpha-split path, after its last shadow ray (rayTrace.compute.ts
 // :870-888): true when the sample is complete (unsplit, zero coverage, or the
 // front path done: radiance, alpha and guides mixed by the coverage);
-// otherwise the back path's result is kept and the front path starts.
-MTD bool finishAlphaSplit(const JobData &J, PathSample &ps, SpectralState &sp) {
+// otherwise the back path's result is kept and the front path starts.  Out of
+// line, as all shading arithmetic is: copies inlined into the kernels could
+// contract its multiply-adds differently, and images are bit-identical across
+// engines.
+static __device__ __noinline__ bool finishAlphaSplit(const JobData &J, PathSample &ps, SpectralState &sp) {
   if (!sp.split || sp.coverage <= 0.0f) return true;
   const float k = sp.coverage;
   auto mix3 = [k](V3 a, V3 b) { return V3{a.x * (1.0f - k) + b.x * k, a.y * (1.0f - k) + b.y * k, a.z * (1.0f - k) + b.z * k}; };
@@ -1724,8 +1727,9 @@ static __device__ __noinline__ bool shadeStepSpectral(Ctx &c, PathSample &ps, Sp
 // End of a spectral wavelength path, after its last NEE shadow ray has been
 // resolved (rayTrace.compute.ts:1036-1053).  Returns true when the sample is
 // complete; its radiance, alpha and guides are then in ps.path / ps.aux for
-// endSample.  Otherwise the next wavelength path starts at event 0.
-MTD bool finishWavelength(const JobData &J, PathSample &ps, SpectralState &sp) {
+// endSample.  Otherwise the next wavelength path starts at event 0.  Out
+// of line like finishAlphaSplit.
+static __device__ __noinline__ bool finishWavelength(const JobData &J, PathSample &ps, SpectralState &sp) {
   if (J.u.dispersion_wavelengths == 1) {
     float scale = sp.dispersivePrimary ? 3.0f : 1.0f;
     ps.path.li = ps.path.li * scale;
