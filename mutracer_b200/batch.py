@@ -237,10 +237,10 @@ class StreamBatch(_JobTable):
 
 # Launch shapes the autotuner tries, in BatchConfig.make's order (block
 # threads, warp tile width, CTAs per SM, items per fetch).  0 keeps the default:
-# one block an SM, all its warps in step; smaller blocks share less of the code
-# they fetch.
+# one block an SM, all its warps in step; smaller blocks (four of 128 threads
+# fit an SM) share less of the code they fetch.
 AUTOTUNE_SPACE = (
-    (0, 8, 0, 1), (0, 8, 0, 2), (0, 4, 0, 1), (0, 16, 0, 1), (0, 32, 0, 1), (128, 8, 8, 1), (128, 8, 4, 1),
+    (0, 8, 0, 1), (0, 8, 0, 2), (0, 4, 0, 1), (0, 16, 0, 1), (0, 32, 0, 1), (128, 8, 4, 1), (64, 8, 8, 1),
 )
 
 

@@ -14,7 +14,7 @@
 
 #include <mutex>
 
-#include "batch_table.cuh"
+#include "pixel_kernels.cuh"
 
 using namespace mt;
 
@@ -88,26 +88,6 @@ cudaError_t scratchAddress(void **out) {
   return cudaSuccess;
 }
 
-// The persistent batched kernel of batch_table.cuh over the fixed scratch.
-template <bool kGpuLayout>
-__global__ void __launch_bounds__(kPixelThreads, 1)
-    k_batch_noalloc(const BatchHeader *__restrict__ header, uint32_t *queue, uint32_t grain, uint32_t *status,
-                    mtc_counters *counters) {
-  Counters cnt;
-  uint32_t paths = 0;
-  batchWorkLoop<kGpuLayout>(header, queue, grain, status, cnt, paths);
-  if (counters) {
-    unsigned mask = __activemask();
-    uint32_t e = __reduce_add_sync(mask, cnt.ext), s = __reduce_add_sync(mask, cnt.shadow);
-    uint32_t p = __reduce_add_sync(mask, paths);
-    if ((threadIdx.x & 31) == uint32_t(__ffs(mask) - 1)) {
-      atomicAdd(&counters->extension_rays, (unsigned long long)e);
-      atomicAdd(&counters->shadow_rays, (unsigned long long)s);
-      atomicAdd(&counters->path_samples, (unsigned long long)p);
-    }
-  }
-}
-
 }  // namespace
 
 // Jobs and launch shape are validated by the same rules as mtc_trace_batch
@@ -148,10 +128,12 @@ extern "C" mt_status mtc_trace_batch_noalloc(const mtc_job_desc *jobs, uint32_t 
   const uint32_t grid = uint32_t(sms) * shape.ctasPerSm;
   const uint32_t flagsUnion = reinterpret_cast<const BatchHeader *>(table)->flagsUnion;
   const BatchHeader *header = (const BatchHeader *)scratch;
-  if (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT)
-    k_batch_noalloc<true><<<grid, shape.blockThreads, 0, cs>>>(header, queue, shape.grain, status_out, counters);
-  else
-    k_batch_noalloc<false><<<grid, shape.blockThreads, 0, cs>>>(header, queue, shape.grain, status_out, counters);
+  const bool gpuLayout = (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  const BatchKernel kernel = shape.shaped ? shapedNoallocKernel(gpuLayout)
+                             : gpuLayout  ? k_batch_noalloc<true, kPixelThreads, 1>
+                                          : k_batch_noalloc<false, kPixelThreads, 1>;
+  kernel<<<grid, shape.blockThreads, rayColumnBytes(shape.blockThreads), cs>>>(header, queue, counters, shape.grain,
+                                                                               status_out);
   e = cudaGetLastError();
   return e == cudaSuccess ? MT_OK : MT_ERROR;
 }

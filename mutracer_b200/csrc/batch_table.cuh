@@ -109,31 +109,39 @@ inline JobData makeJob(const mtc_scene_view *scene, const mtc_camera_uniform *ca
   return J;
 }
 
-// Threads per block the megakernels are compiled for and run with by default:
-// one block fills an SM at 64 registers, its 32 warps in step (tracePixels).
-// 512 threads at 128 registers: 20 % faster on glass and on 256x256 previews,
-// 10 to 30 % slower on the Cornell, instanced and batched runs.
+// Threads per block the megakernels run with by default: one block fills an SM
+// at 64 registers, its 32 warps in step (tracePixels).
 constexpr uint32_t kPixelThreads = 1024;
+
+// Blocks of the size a host asks for (32 to 128 threads) run kernels compiled
+// for four of 128 threads an SM, at 128 registers.  Smaller blocks share less of
+// the code they fetch and gain more from registers than from more warps: 8
+// uneven jobs of instanced scenes 176 ms, two samples of a 512x512 Cornell box
+// 5.7 ms; eight blocks at 64 registers 186 and 7.1, sixteen at 32 registers 186
+// and 7.4 (free-running warps with one thread per pixel: 227 and 8.5).
+constexpr uint32_t kShapedThreads = 128, kShapedBlocks = 4;
 
 struct BatchShape {
   uint32_t blockThreads, tileW, tileH, ctasPerSm, grain;
+  bool shaped;  // block size given: kShapedThreads at most
 };
 // Resolves a (possibly NULL) mtc_batch_config to launch parameters; false for
 // out-of-range values.
 inline bool batchShape(const mtc_batch_config *c, BatchShape &out) {
-  out = BatchShape{kPixelThreads, 8u, 4u, 1u, 1u};
+  out = BatchShape{kPixelThreads, 8u, 4u, 1u, 1u, false};
   if (!c) return true;
   if (c->struct_size != sizeof(mtc_batch_config)) return false;
   if (c->block_threads) {
     if (c->block_threads > 128u || c->block_threads % 32u) return false;
     out.blockThreads = c->block_threads;
+    out.ctasPerSm = kShapedThreads * kShapedBlocks / c->block_threads;
+    out.shaped = true;
   }
   if (c->tile_width) {
     if (c->tile_width > 32u || (32u % c->tile_width)) return false;
     out.tileW = c->tile_width;
     out.tileH = 32u / c->tile_width;
   }
-  out.ctasPerSm = kPixelThreads / out.blockThreads;
   if (c->ctas_per_sm) {
     if (c->ctas_per_sm > 32u) return false;
     out.ctasPerSm = c->ctas_per_sm;
@@ -241,9 +249,8 @@ struct TableClaims {
 template <bool kGpuLayout>
 __device__ __forceinline__ void batchWorkLoop(const BatchHeader *__restrict__ header, uint32_t *queue, uint32_t grain,
                                               uint32_t *status, Counters &cnt, uint32_t &paths) {
-  __shared__ float columns[kPixelThreads / 32][9 * 32];
   TableClaims claims(header, queue, status, grain);
-  tracePixels<kGpuLayout>(claims, cnt, paths, &columns[threadIdx.x / 32u][threadIdx.x & 31u]);
+  tracePixels<kGpuLayout>(claims, cnt, paths);
 }
 
 }  // namespace mt

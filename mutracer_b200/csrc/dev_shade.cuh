@@ -1825,8 +1825,11 @@ static __device__ __noinline__ void endSample(const JobData &J, uint32_t idx, co
 // The megakernels' work loop, run by all threads of a block together.  Each
 // lane owns a pixel of a job at a time: all its samples in order, each
 // accumulated before the next begins (the same sums as as many separate
-// dispatches), then the next pixel that `claims` gives it.  `column` is the
-// lane's column of its warp's world-space rays in shared memory.
+// dispatches), then the next pixel that `claims` gives it.  The launch provides
+// rayColumnBytes(threads) of shared memory: a column a lane, of the world-space
+// ray that its warp traces.  (Sized for 1,024 threads whatever the block, it
+// took the L1 from the spilled state of small blocks: 24x24 pixels of the
+// Cornell box, 4 samples, 1.95 ms against 1.57.)
 //
 // Instruction fetch is what bounds these kernels once each warp runs on its
 // own: 64 warps an SM at different places of the shading code fetch it apart.
@@ -1837,8 +1840,13 @@ static __device__ __noinline__ void endSample(const JobData &J, uint32_t idx, co
 // claims.next(wants, job, x, y, samples), called by whole warps, gives a lane
 // that wants one its next pixel with samples to add (samples stays 0: none is
 // left).
+constexpr uint32_t kRayColumn = 9;  // origin, direction, inverse direction
+constexpr size_t rayColumnBytes(uint32_t threads) { return size_t(threads) * kRayColumn * sizeof(float); }
+
 template <bool kGpuLayout, class Claims>
-MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths, float *column) {
+MTD void tracePixels(Claims &claims, Counters &cnt, uint32_t &paths) {
+  extern __shared__ float rayColumns[];
+  float *const column = rayColumns + threadIdx.x / 32u * (32u * kRayColumn) + (threadIdx.x & 31u);
   Ctx c{nullptr, Sampler(), BsdfContext(), ShadowQuery()};
   const JobData *job = nullptr;
   PathSample ps;  // ps and sp hold a path, and c its job, while left > 0

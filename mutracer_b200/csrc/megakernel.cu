@@ -16,27 +16,12 @@
 #include <cstring>
 #include <vector>
 
-#include "batch_table.cuh"
 #include "js_minmax.h"
+#include "pixel_kernels.cuh"
 
 using namespace mt;
 
 namespace {
-
-__device__ __forceinline__ void flushCounters(const Counters &cnt, uint32_t paths, mtc_counters *out) {
-  if (!out) return;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(&out->kernel_launches, 1ull);
-  unsigned mask = __activemask();
-  uint32_t e = __reduce_add_sync(mask, cnt.ext);
-  uint32_t s = __reduce_add_sync(mask, cnt.shadow);
-  uint32_t p = __reduce_add_sync(mask, paths);
-  int leader = __ffs(mask) - 1;
-  if ((threadIdx.x & 31) == leader) {
-    atomicAdd(&out->extension_rays, (unsigned long long)e);
-    atomicAdd(&out->shadow_rays, (unsigned long long)s);
-    atomicAdd(&out->path_samples, (unsigned long long)p);
-  }
-}
 
 // The pixels of one image in the order of its 8x4 tiles: the grid's blocks take
 // turns at runs of `run` of them, which a block's lanes claim one by one.  Of
@@ -99,25 +84,13 @@ constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
 template <bool kGpuLayout>
 __global__ void __launch_bounds__(kPixelThreads, 1)
     k_trace(const __grid_constant__ JobData J, uint32_t samples, uint32_t lanes, mtc_counters *counters) {
-  __shared__ float columns[kPixelThreads / 32][9 * 32];
   __shared__ uint32_t cursor;
   if (threadIdx.x == 0) cursor = 0;
   __syncthreads();
   Counters cnt;
   uint32_t paths = 0;
   ImageClaims claims{J, samples, &cursor, blockDim.x / 32u * lanes, lanes};
-  tracePixels<kGpuLayout>(claims, cnt, paths, &columns[threadIdx.x / 32u][threadIdx.x & 31u]);
-  flushCounters(cnt, paths, counters);
-}
-
-// Persistent batched kernel over a job table (batch_table.cuh).
-template <bool kGpuLayout>
-__global__ void __launch_bounds__(kPixelThreads, 1)
-    k_batch(const BatchHeader *__restrict__ header, uint32_t *queue, mtc_counters *counters, uint32_t grain,
-            uint32_t *status) {
-  Counters cnt;
-  uint32_t paths = 0;
-  batchWorkLoop<kGpuLayout>(header, queue, grain, status, cnt, paths);
+  tracePixels<kGpuLayout>(claims, cnt, paths);
   flushCounters(cnt, paths, counters);
 }
 
@@ -356,7 +329,7 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
     grid = uint32_t(std::max<uint64_t>(1, units));
   }
   auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_trace<true> : k_trace<false>;
-  kernel<<<grid, warps * 32u, 0, (cudaStream_t)stream>>>(J, samples, lanes, counters);
+  kernel<<<grid, warps * 32u, rayColumnBytes(warps * 32u), (cudaStream_t)stream>>>(J, samples, lanes, counters);
   return cudaStatus(cudaGetLastError());
 }
 
@@ -444,12 +417,12 @@ mt_status launchBatch(const void *table, uint32_t capacity, const BatchShape &sh
   uint32_t grid = uint32_t(sms) * shape.ctasPerSm;
   // The host copy of the header decides the BLAS-layout specialisation.
   uint32_t flagsUnion = static_cast<const BatchHeader *>(table)->flagsUnion;
-  if (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT)
-    k_batch<true><<<grid, shape.blockThreads, 0, st>>>((const BatchHeader *)scratch, queue, counters, shape.grain,
-                                                       status);
-  else
-    k_batch<false><<<grid, shape.blockThreads, 0, st>>>((const BatchHeader *)scratch, queue, counters, shape.grain,
-                                                        status);
+  const bool gpuLayout = (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  const BatchKernel kernel = shape.shaped ? shapedBatchKernel(gpuLayout)
+                             : gpuLayout  ? k_batch<true, kPixelThreads, 1>
+                                          : k_batch<false, kPixelThreads, 1>;
+  kernel<<<grid, shape.blockThreads, rayColumnBytes(shape.blockThreads), st>>>((const BatchHeader *)scratch, queue,
+                                                                               counters, shape.grain, status);
   return cudaStatus(cudaGetLastError());
 }
 

@@ -65,3 +65,29 @@ def test_unlike_jobs_agree_in_the_other_engines(cuda, scenes, alone):
     torch.cuda.synchronize()
     for want, a, b in zip(alone, jobs, fixed):
         assert _same(want.acc, a.acc) and _same(want.acc, b.acc)
+
+
+@pytest.mark.parametrize("layout", [0, 2])
+@pytest.mark.parametrize("threads", [32, 64, 96, 128])
+def test_blocks_of_a_given_size_trace_both_layouts(cuda, threads, layout):
+    """A host's own block sizes run kernels of their own, in both batched
+    entry points: ragged images, with the default and with more blocks an SM
+    than fit one."""
+    import torch
+    host = scene.SceneHost("instanced_spheres", 75, 46, 3, (24, 3, 4, 64, 2))
+    if layout:
+        host.set_blas_layout(layout)
+    dev = scene.DeviceScene(host, cuda)
+    want = batch.RenderJob(dev, 2, device=cuda)
+    want.render_alone()
+    for ctas in (0, 32):
+        cfg = abi.BatchConfig.make(threads, 4, ctas, 2)
+        job, fixed = batch.RenderJob(dev, 2, device=cuda), batch.RenderJob(dev, 2, device=cuda)
+        b = batch.Batch(1, cfg, cuda)
+        b.set_jobs([job])
+        b.launch()
+        descs = (abi.JobDesc * 1)(fixed.desc(2))
+        abi.check(abi.lib().mtc_trace_batch_noalloc(descs, 1, C.byref(cfg), None, None,
+                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+        assert _same(want.acc, job.acc) and _same(want.acc, fixed.acc), ctas
