@@ -14,7 +14,8 @@ OUT = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT, "libmutracer_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU = ["megakernel.cu", "pixel_kernels_r128.cu", "batch_noalloc.cu", "wavefront.cu", "bvh_build.cu", "blas_refit.cu"]
+CU = ["megakernel.cu", "pixel_kernels_r128.cu", "pixel_kernels_r255.cu", "batch_noalloc.cu", "wavefront.cu",
+      "bvh_build.cu", "blas_refit.cu"]
 CPP = ["scene_prep.cpp", "host_api.cpp", "context.cpp", "sizes.cpp", "descriptor.cpp"]
 ENERGY_LUT = os.path.join(CSRC, "openpbr_energy_lut.f32")
 

@@ -23,76 +23,17 @@ using namespace mt;
 
 namespace {
 
-// The pixels of one image in the order of its 8x4 tiles: the grid's blocks take
-// turns at runs of `run` of them, which a block's lanes claim one by one.  Of
-// each warp `lanes` lanes ask: a small image is spread over all warps an SM
-// holds, a few lanes in each, rather than over full warps of a few.
-struct ImageClaims {
-  const JobData &J;
-  uint32_t samples;
-  uint32_t *cursor;  // shared: the block's next pixel
-  uint32_t run, lanes;
-  bool exhausted = false;
-
-  MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &left) {
-    const uint32_t lane = threadIdx.x & 31u, tilesX = (J.width + 7u) / 8u;
-    const uint64_t units = uint64_t(tilesX) * ((J.height + 3u) / 4u) * 32u;
-    wants = wants && lane < lanes;
-    unsigned asking = __ballot_sync(0xffffffffu, wants);
-    while (asking && !exhausted) {
-      uint32_t k = 0;
-      if (lane == 0) k = atomicAdd(cursor, uint32_t(__popc(asking)));
-      k = __shfl_sync(0xffffffffu, k, 0) + __popc(asking & ((1u << lane) - 1u));
-      const uint64_t u = (uint64_t(k / run) * gridDim.x + blockIdx.x) * run + k % run;
-      if (wants && u < units) {
-        const uint32_t tile = uint32_t(u / 32u), in = uint32_t(u % 32u);
-        x = tile % tilesX * 8u + in % 8u;
-        y = tile / tilesX * 4u + in / 8u;
-        if (x < J.width && y < J.height) {
-          job = &J;
-          left = samples;
-          wants = false;
-        }
-      }
-      // Pixels ascend with the cursor: none is left once one lies past the
-      // image.
-      exhausted = __any_sync(0xffffffffu, wants && u >= units);
-      asking = __ballot_sync(0xffffffffu, wants);
-    }
-  }
-};
-
 // Small images: up to 256 pixels an SM go to 8 warps of one block, a few lanes
-// each.  Few lanes mean little divergence: 61x47 pixels of the instanced scene
-// take 4.7 ms that way, 9.3 in full warps, 13.0 with one thread per pixel in
-// free-running blocks; 128x72 of glass 11.0, 17.1 and 17.8.  (16 warps: 5.2 and
-// 12.3, and 5 % slower on a 256x256 Cornell box.)  Where paths hardly diverge
-// the block's meetings cost more than that gives: 61x47 of the Cornell box 1.96
-// against 1.60 ms.  Up to kAlonePixels an SM, each pixel gets a block of one
-// warp: nothing to share, no one to wait for (17x13 pixels x 16 samples of the
-// Cornell box 5.1 ms, in pairs 5.9).
+// each.  Few lanes mean little divergence (61x47 pixels, ms with 8 warps of few
+// lanes, 4 of more, full warps in blocks of 1 and of 8: the instanced scene, 4
+// samples, 1.71, 1.92, 2.53 and 3.04; glass, 2 samples, 9.1, 10.4, 12.6 and 14.9;
+// the Cornell box, 4 samples, 1.11, 1.10, 1.17 and 1.28; with one thread per
+// pixel in free-running blocks 4.7, 24.9 and 1.46).  Up to kAlonePixels an SM,
+// each pixel gets a block of one warp and waits for no other, which pays where
+// paths diverge most (24x24 pixels, alone and four to a block: glass 9.7 and
+// 10.6 ms, the instanced scene 1.12 and 1.03, the Cornell box 1.29 and 0.88;
+// free-running threads 43, 4.4 and 1.37).
 constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
-
-// The plain megakernel.  Bound by instruction fetch and by the latency of its
-// spilled state; with the 32 warps of an SM's block in step 4 samples of the
-// 4M-triangle instanced scene at 960x540 take 29.2 ms (64 free-running warps
-// an SM with one thread per pixel: 67.2), 8 of the Cornell box at 512x512 13.8
-// (29.6), one of the glass scene at 640x360 24.0 (85.2), one of a 256x256
-// Cornell box 1.1 (2.5).  Free-running warps that trace and shade together,
-// or that shade once 8, 12 or 20 lanes wait, are slower than one thread per
-// pixel: it is the fetches shared by the block that pay.
-template <bool kGpuLayout>
-__global__ void __launch_bounds__(kPixelThreads, 1)
-    k_trace(const __grid_constant__ JobData J, uint32_t samples, uint32_t lanes, mtc_counters *counters) {
-  __shared__ uint32_t cursor;
-  if (threadIdx.x == 0) cursor = 0;
-  __syncthreads();
-  Counters cnt;
-  uint32_t paths = 0;
-  ImageClaims claims{J, samples, &cursor, blockDim.x / 32u * lanes, lanes};
-  tracePixels<kGpuLayout>(claims, cnt, paths);
-  flushCounters(cnt, paths, counters);
-}
 
 __global__ void k_sample_maps(const __grid_constant__ DevScene s, const int32_t *indices, const float2 *uvs,
                               uint32_t count, float4 *out) {
@@ -328,7 +269,14 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
     warps = lanes = 1;
     grid = uint32_t(std::max<uint64_t>(1, units));
   }
-  auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_trace<true> : k_trace<false>;
+  // The most registers that blocks of so many warps leave room for: 24x24 pixels
+  // of the Cornell box, 4 samples, 1.29 ms (1.57 at 64 registers); 256x256, one
+  // sample, 0.80 (0.96); 61x47 of glass, 2 samples, 9.1 (11.9).
+  const bool gpuLayout = (scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  const TraceKernel kernel = warps <= 8u    ? traceKernel256(gpuLayout)
+                             : warps <= 16u ? traceKernel512(gpuLayout)
+                             : gpuLayout    ? k_trace<true, kPixelThreads>
+                                            : k_trace<false, kPixelThreads>;
   kernel<<<grid, warps * 32u, rayColumnBytes(warps * 32u), (cudaStream_t)stream>>>(J, samples, lanes, counters);
   return cudaStatus(cudaGetLastError());
 }

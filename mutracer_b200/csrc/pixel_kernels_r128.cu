@@ -3,6 +3,8 @@
 
 namespace mt {
 
+TraceKernel traceKernel512(bool gpuLayout) { return gpuLayout ? k_trace<true, 512> : k_trace<false, 512>; }
+
 BatchKernel shapedBatchKernel(bool gpuLayout) {
   return gpuLayout ? k_batch<true, kShapedThreads, kShapedBlocks> : k_batch<false, kShapedThreads, kShapedBlocks>;
 }

@@ -91,3 +91,23 @@ def test_blocks_of_a_given_size_trace_both_layouts(cuda, threads, layout):
                                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)))
         torch.cuda.synchronize()
         assert _same(want.acc, job.acc) and _same(want.acc, fixed.acc), ctas
+
+
+@pytest.mark.parametrize("layout", [0, 2])
+@pytest.mark.parametrize("size", [(24, 24), (199, 150), (251, 240), (300, 291), (1007, 701)])
+def test_plain_kernels_of_every_block_size(cuda, size, layout):
+    """One warp a pixel, then blocks of up to 8, 16 and 32 warps and several a
+    multiprocessor: the image of the batched kernel, every pixel once."""
+    import torch
+    host = scene.SceneHost("instanced_spheres", *size, 3, (24, 3, 4, 64, 2))
+    if layout:
+        host.set_blas_layout(layout)
+    dev = scene.DeviceScene(host, cuda)
+    plain, job = batch.RenderJob(dev, 2, device=cuda), batch.RenderJob(dev, 2, device=cuda)
+    plain.render_alone()
+    b = batch.Batch(1, device=cuda)
+    b.set_jobs([job])
+    b.launch()
+    torch.cuda.synchronize()
+    assert (plain.acc.normal[:, 3] == 2).all()
+    assert _same(plain.acc, job.acc)
