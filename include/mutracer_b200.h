@@ -259,7 +259,9 @@ uint32_t mtc_abi_version(void);
  * y < output_size.y traces one path sample and adds to `out`.  The per-pixel
  * sample index is read from out->normal[idx].w + sample_sequence_offset,
  * exactly as rayTrace.compute.ts:1187-1193.  Replaces the per-sample dispatch
- * loop of native/host/src/lib.rs:1506-1560.  counters may be NULL. */
+ * loop of native/host/src/lib.rs:1506-1560.  counters may be NULL.  A block of
+ * the kernel fills a multiprocessor and leaves it after all samples of about
+ * 4,096 pixels; a stream of higher priority is let in as blocks leave. */
 mt_status mtc_trace_samples(const mtc_scene_view *scene,
                             const mtc_camera_uniform *camera,
                             const mtc_trace_uniform *uniform,

@@ -35,6 +35,22 @@ namespace {
 // free-running threads 43, 4.4 and 1.37).
 constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
 
+// Large images: a block holds its SM until it ends, and a stream of higher
+// priority is let in only then, so a block gets about kBlockPixels pixels (a pick
+// during a 1080p render of the instanced scene, 4 samples, 91 ms, waits 20 ms at
+// most; in a single block an SM 68 ms, with free-running blocks of 128 threads
+// 20).  That costs the lanes that are idle at the end of each block: 46.1 against
+// 45.7 ms for 2 samples of that scene, 16.0 against 15.2 of the Cornell box;
+// blocks of 3,072 pixels 49.7 and 17.6, of 2,048 46.7 and 18.4.
+constexpr uint64_t kBlockPixels = 4096;
+// A single block an SM takes turns at runs of kRunPixels pixels, which leaves no
+// two blocks more than one run apart (runs of 1,024: up to 1,024 pixels apart;
+// 801x601, 2 samples, Cornell box 5.20 against 5.79 ms, instanced scene 8.55 and
+// 9.26; one sample of 401x378 1.47 and 1.68; runs of 256 and 32 within 3 % of
+// 64).  With blocks to follow, runs of a pixel a lane keep neighbours together:
+// 46.1 against 49.5 ms with runs of 128 in the 1080p render above.
+constexpr uint32_t kRunPixels = 64;
+
 __global__ void k_sample_maps(const __grid_constant__ DevScene s, const int32_t *indices, const float2 *uvs,
                               uint32_t count, float4 *out) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,12 +279,16 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
   const uint64_t perSm = std::max<uint64_t>(1, (units + uint64_t(sms) - 1) / uint64_t(sms));
   uint32_t warps = uint32_t(std::min<uint64_t>(
       kPixelThreads / 32, perSm <= kSpreadWarps * 32u ? std::min<uint64_t>(kSpreadWarps, perSm) : (perSm + 31) / 32));
-  uint32_t lanes = uint32_t(std::min<uint64_t>(32, (perSm + warps - 1) / warps));
+  ImageSplit split;
+  split.lanes = uint32_t(std::min<uint64_t>(32, (perSm + warps - 1) / warps));
   uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms), units)));
   if (perSm <= kAlonePixels) {
-    warps = lanes = 1;
+    warps = split.lanes = 1;
     grid = uint32_t(std::max<uint64_t>(1, units));
   }
+  const uint32_t turns = uint32_t(std::max<uint64_t>(1, perSm / kBlockPixels));
+  split.run = turns == 1 && perSm > kPixelThreads ? kRunPixels : warps * split.lanes;
+  grid *= turns;
   // The most registers that blocks of so many warps leave room for: 24x24 pixels
   // of the Cornell box, 4 samples, 1.29 ms (1.57 at 64 registers); 256x256, one
   // sample, 0.80 (0.96); 61x47 of glass, 2 samples, 9.1 (11.9).
@@ -277,7 +297,7 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
                              : warps <= 16u ? traceKernel512(gpuLayout)
                              : gpuLayout    ? k_trace<true, kPixelThreads>
                                             : k_trace<false, kPixelThreads>;
-  kernel<<<grid, warps * 32u, rayColumnBytes(warps * 32u), (cudaStream_t)stream>>>(J, samples, lanes, counters);
+  kernel<<<grid, warps * 32u, rayColumnBytes(warps * 32u), (cudaStream_t)stream>>>(J, samples, split, counters);
   return cudaStatus(cudaGetLastError());
 }
 

@@ -34,23 +34,26 @@ __device__ __forceinline__ void flushCounters(const Counters &cnt, uint32_t path
 // turns at runs of `run` of them, which a block's lanes claim one by one.  Of
 // each warp `lanes` lanes ask: a small image is spread over all warps an SM
 // holds, a few lanes in each, rather than over full warps of a few.
+struct ImageSplit {
+  uint32_t run, lanes;
+};
 struct ImageClaims {
   const JobData &J;
   uint32_t samples;
   uint32_t *cursor;  // shared: the block's next pixel
-  uint32_t run, lanes;
+  ImageSplit split;
   bool exhausted = false;
 
   MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &left) {
     const uint32_t lane = threadIdx.x & 31u, tilesX = (J.width + 7u) / 8u;
     const uint64_t units = uint64_t(tilesX) * ((J.height + 3u) / 4u) * 32u;
-    wants = wants && lane < lanes;
+    wants = wants && lane < split.lanes;
     unsigned asking = __ballot_sync(0xffffffffu, wants);
     while (asking && !exhausted) {
       uint32_t k = 0;
       if (lane == 0) k = atomicAdd(cursor, uint32_t(__popc(asking)));
       k = __shfl_sync(0xffffffffu, k, 0) + __popc(asking & ((1u << lane) - 1u));
-      const uint64_t u = (uint64_t(k / run) * gridDim.x + blockIdx.x) * run + k % run;
+      const uint64_t u = (uint64_t(k / split.run) * gridDim.x + blockIdx.x) * split.run + k % split.run;
       if (wants && u < units) {
         const uint32_t tile = uint32_t(u / 32u), in = uint32_t(u % 32u);
         x = tile % tilesX * 8u + in % 8u;
@@ -79,18 +82,18 @@ struct ImageClaims {
 // pixel: it is the fetches shared by the block that pay.
 template <bool kGpuLayout, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_trace(const __grid_constant__ JobData J, uint32_t samples, uint32_t lanes, mtc_counters *counters) {
+    k_trace(const __grid_constant__ JobData J, uint32_t samples, ImageSplit split, mtc_counters *counters) {
   __shared__ uint32_t cursor;
   if (threadIdx.x == 0) cursor = 0;
   __syncthreads();
   Counters cnt;
   uint32_t paths = 0;
-  ImageClaims claims{J, samples, &cursor, blockDim.x / 32u * lanes, lanes};
+  ImageClaims claims{J, samples, &cursor, split};
   tracePixels<kGpuLayout>(claims, cnt, paths);
   flushCounters(cnt, paths, counters);
 }
 
-using TraceKernel = void (*)(const JobData, uint32_t, uint32_t, mtc_counters *);
+using TraceKernel = void (*)(const JobData, uint32_t, ImageSplit, mtc_counters *);
 // The kernels for blocks of up to 512 and 256 threads.
 TraceKernel traceKernel512(bool gpuLayout);
 TraceKernel traceKernel256(bool gpuLayout);

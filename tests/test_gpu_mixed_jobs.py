@@ -94,7 +94,7 @@ def test_blocks_of_a_given_size_trace_both_layouts(cuda, threads, layout):
 
 
 @pytest.mark.parametrize("layout", [0, 2])
-@pytest.mark.parametrize("size", [(24, 24), (199, 150), (251, 240), (300, 291), (1007, 701)])
+@pytest.mark.parametrize("size", [(24, 24), (199, 150), (251, 240), (300, 291), (1007, 701), (1403, 901)])
 def test_plain_kernels_of_every_block_size(cuda, size, layout):
     """One warp a pixel, then blocks of up to 8, 16 and 32 warps and several a
     multiprocessor: the image of the batched kernel, every pixel once."""
