@@ -7,7 +7,8 @@
 //                  for its lanes, which run every sample of their pixel in
 //                  order, so a job's image is bit-identical alone and in a
 //                  batch (mixed jobs: 91 ms, with free-running warps 225);
-//  - k_first_hit:  querySceneSoftware (intersect.wgsl.ts:660-684);
+//  - k_first_hit, k_first_hit_queue: querySceneSoftware
+//                  (intersect.wgsl.ts:660-684);
 //  - k_sample_maps: raw material-map lookups (sampleMap) for parity checks;
 //  - k_refit_*:    TLAS refit (bvhAccel.ts:579-740) on the device.
 #include <cuda_runtime.h>
@@ -59,11 +60,8 @@ __global__ void k_sample_maps(const __grid_constant__ DevScene s, const int32_t 
   out[i] = sampleMap(s, indices[i], V2{uv.x, uv.y});
 }
 
-// querySceneSoftware for `raysPerWarp` consecutive rays a warp, through the
-// traversal of the wavefront engine: a lane whose ray is finished takes the
-// warp's next one.  Latency- and divergence-bound: 1M scattered rays over the
-// 4M-triangle instanced scene take 2.80 ms, with one ray a thread for good
-// 5.56 ms; 33 rays 17 us against 24 us, launch included.
+// querySceneSoftware (intersect.wgsl.ts:660-684) for a buffer of rays, through
+// the traversal of the wavefront engine.
 struct FirstHitSource {
   const DevScene &s;
   const float4 *rays;
@@ -111,22 +109,75 @@ struct FirstHitSource {
 };
 
 constexpr int kHitThreads = 128;
-// Up to this many vec4 (the 47 of the Cornell box; the smallest mesh scenes have
-// thousands) a BVH counts as small: 832,000 rays 260 us in step, 324 us with
-// lanes taking rays as they finish, 249 us with one ray a thread.
-constexpr uint64_t kUniformNodes = 1024;
-template <bool kGpuLayout>
+
+// A lane traces one ray, `raysPerWarp` of them a warp.  Bound by the latency of
+// the node loads, and by divergence once warps are full.  With a ray a warp
+// (kAlone) the lane asks no other what comes next: one ray of the 4M-triangle
+// instanced scene 82 us, 1,000 rays 110; as queries of k_first_hit_queue 98 and
+// 136; with a thread a ray and full warps 85 and 463.  In a small scene a queue's
+// fetches cost bulk queries more than its lanes gain: 1M rays of the Cornell box
+// 292 us, queued 328, with the thread-a-ray traversal 314.
+template <bool kGpuLayout, bool kAlone>
 __global__ void __launch_bounds__(kHitThreads, 5)
     k_first_hit(const __grid_constant__ DevScene s, int32_t blasBase, int32_t isEmpty, const float4 *rays,
-                uint32_t count, uint32_t raysPerWarp, uint32_t refillLanes, mtc_hit *hits) {
+                uint32_t count, uint32_t raysPerWarp, mtc_hit *hits) {
+  __shared__ float columns[kHitThreads / 32][9][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x / 32u;
+  const uint64_t t = (uint64_t(blockIdx.x) * (kHitThreads / 32) + warp) * raysPerWarp + lane;
+  FirstHitSource src{s, rays, hits, blasBase, isEmpty != 0, 0u};
+  int2 stack[kTraversalStackEntries];
+  RayTraversal<false, kGpuLayout> rt;
+  rt.stack = stack;
+  rt.finish(rt.kIdle);
+  RayQuery q;
+  if (lane < raysPerWarp && t < count && src.read(uint32_t(t), q)) {
+    const V3 inv = traversalInverse(q.d);
+    if (entersScene(s, q.o, inv, q.limit))
+      rt.begin(s, blasBase, &columns[warp][0][lane], q.o, q.d, inv, q.limit, q.tri, q.ins, q.doubleSided);
+    else
+      src.missed(q);
+  }
+  if (kAlone) {
+    while (rt.state < rt.kDone) {
+      if (rt.atLeaf()) rt.leaf();
+      else if (rt.atInstances()) rt.enter();
+      else do rt.visit(); while (rt.atNode());
+    }
+  } else {
+    __syncwarp();
+    while (__any_sync(0xffffffffu, rt.state < rt.kDone)) rt.advance(8u, 1u);
+  }
+  if (rt.state == rt.kDone) src.done(rt, uint32_t(t));
+}
+
+// `raysPerWarp` consecutive rays a warp, whose lanes take the next one as they
+// finish: 1M scattered rays over the 4M-triangle instanced scene take 2.65 ms
+// (a ray a lane 2.79, with full warps of the former traversal 5.31), over glass
+// spheres 460 us (497, 654).
+template <bool kGpuLayout>
+__global__ void __launch_bounds__(kHitThreads, 5)
+    k_first_hit_queue(const __grid_constant__ DevScene s, int32_t blasBase, int32_t isEmpty, const float4 *rays,
+                      uint32_t count, uint32_t raysPerWarp, mtc_hit *hits) {
   __shared__ WarpRays warpRays[kHitThreads / 32];
   const uint64_t first = (uint64_t(blockIdx.x) * (kHitThreads / 32) + threadIdx.x / 32u) * raysPerWarp;
   if (first >= count) return;
   const uint32_t end = uint32_t(min(uint64_t(count), first + raysPerWarp));
   FirstHitSource src{s, rays, hits, blasBase, isEmpty != 0, uint32_t(first)};
-  traceQueue<false, kGpuLayout, false>(src, end, min(32u, raysPerWarp), raysPerWarp >= kDenseRays ? kNodeLanes : 1u,
-                                       refillLanes, 8u, warpRays[threadIdx.x / 32u]);
+  traceQueue<false, kGpuLayout, false>(src, end, 32u, raysPerWarp >= kDenseRays ? kNodeLanes : 1u, 4u, 8u,
+                                       warpRays[threadIdx.x / 32u]);
 }
+
+// Queues pay where rays differ in length and there are many: with kQueueRays a
+// warp and three waves of warps (200,000 rays, 23 a warp that way: the
+// instanced scene 935 us, a ray a lane 720; glass 196 and 155).  In BVHs of few
+// vec4 rays take much the same steps (1M rays a lane and queued, us: 1,187 vec4
+// 560 and 643, 2,127 vec4 727 and 753; 9,793 vec4 of glass 497 and 460).
+constexpr uint64_t kQueueRays = 64, kQueueWarps = 5 * (kHitThreads / 32) * 3;  // of an SM
+constexpr uint64_t kQueueNodes = 4096;
+// Warps an SM among which fewer rays are spread before a warp gets a second one:
+// 20,000 rays (12 a warp) of the instanced scene 264 us at 8 a warp, 298 at 16,
+// 331 at 32; of one sphere 38.6, 40.3, 41.9.
+constexpr uint64_t kSpreadHitWarps = 12;
 
 // read_average (native/host/src/lib.rs:343-364): each f32 of an accumulation
 // buffer divided by the completed sample count; any non-finite result raises
@@ -308,19 +359,17 @@ mt_status mtc_query_first_hit(const mtc_scene_view *scene, const float *rays, ui
   int device = 0, sms = 148;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  // A few rays: one a warp, which then waits for no other.  Many: up to 256 a
-  // warp, as long as there are enough warps left to fill the SMs three times.
-  // In a small BVH rays take much the same steps: 32 a warp that start and
-  // finish together, once there is a warp of them for every scheduler.
-  const bool together = scene->bvh_vec4_count <= kUniformNodes;
-  const uint64_t warps = uint64_t(sms) * (together ? 4u : 5u * (kHitThreads / 32) * 3u);
-  const uint32_t perWarp = uint32_t(std::min<uint64_t>(together ? 32u : 256u, (count + warps - 1u) / warps));
+  const bool gpuLayout = (scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  const bool queue = scene->bvh_vec4_count > kQueueNodes && count >= uint64_t(sms) * kQueueWarps * kQueueRays;
+  const uint64_t warps = uint64_t(sms) * (queue ? kQueueWarps : kSpreadHitWarps);
+  const uint32_t perWarp = uint32_t(std::min<uint64_t>(queue ? 256u : 32u, (count + warps - 1u) / warps));
   const uint32_t perBlock = perWarp * (kHitThreads / 32);
   const uint32_t grid = uint32_t((uint64_t(count) + perBlock - 1u) / perBlock);
-  const int32_t blasBase = scene->blas_offset;
-  auto kernel = scene->flags & MTC_SCENE_BLAS_GPU_LAYOUT ? k_first_hit<true> : k_first_hit<false>;
-  kernel<<<grid, kHitThreads, 0, (cudaStream_t)stream>>>(toDev(scene), blasBase, scene->instance_count == 0,
-                                                         (const float4 *)rays, count, perWarp, together ? 32u : 4u, hits);
+  auto kernel = queue          ? (gpuLayout ? k_first_hit_queue<true> : k_first_hit_queue<false>)
+                : perWarp > 1u ? (gpuLayout ? k_first_hit<true, false> : k_first_hit<false, false>)
+                               : (gpuLayout ? k_first_hit<true, true> : k_first_hit<false, true>);
+  kernel<<<grid, kHitThreads, 0, (cudaStream_t)stream>>>(toDev(scene), scene->blas_offset, scene->instance_count == 0,
+                                                         (const float4 *)rays, count, perWarp, hits);
   return cudaStatus(cudaGetLastError());
 }
 

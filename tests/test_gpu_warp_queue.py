@@ -29,6 +29,26 @@ def test_first_hits_at_batch_edges(cuda, count, layout):
     assert (same | tie).all()
 
 
+@pytest.mark.parametrize("layout", [0, 2])
+def test_bulk_first_hits_match_smaller_calls(cuda, layout):
+    """Ray counts and scenes on either side of the rules that hand rays to lanes
+    one by one or for good: the same bits as in calls of a few thousand rays."""
+    import torch
+    host = scene.SceneHost("instanced_spheres", 32, 32, 3, (24, 6, 6, 64, 2))
+    few = scene.SceneHost("cornell", 32, 32, 3)
+    if layout:
+        host.set_blas_layout(layout)
+        few.set_blas_layout(layout)
+    for h in (host, few):
+        dev = scene.DeviceScene(h, cuda)
+        assert (dev.view.bvh_vec4_count > 4096) == (h is host)
+        sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+        rays = torch.from_numpy(oracle_lib.seeded_rays(h, sms * 60 * 64 + 37, seed=5)).to(cuda)
+        part = torch.cat([trace.query_first_hit(dev, r) for r in rays.split(3001)])
+        for count in (len(rays), sms * 60 * 64 - 1, sms * 12 * 3 + 1, sms * 12):
+            assert torch.equal(trace.query_first_hit(dev, rays[:count].contiguous()), part[:count]), (count, layout)
+
+
 def _same(a, b):
     import torch
     return all(torch.equal(getattr(a, k), getattr(b, k)) for k in ("color", "normal", "albedo", "catcher"))
