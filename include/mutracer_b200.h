@@ -397,7 +397,8 @@ typedef struct mtc_job_desc {
 typedef struct mtc_batch_config {
   uint32_t struct_size;
   uint32_t block_threads;    /* threads per CTA: 32, 64, 96 or 128 (default: one CTA
-                                of 1,024 that fills its SM) */
+                                of 1,024 that fills its SM,
+                                or smaller ones for tables of few pixels) */
   uint32_t tile_width;       /* warp tile width in pixels: 1, 2, 4, 8, 16 or 32;
                                 height = 32 / width (default 8, an 8x4 tile) */
   uint32_t ctas_per_sm;      /* grid = SM count * ctas_per_sm (default: as many as an

@@ -125,15 +125,16 @@ extern "C" mt_status mtc_trace_batch_noalloc(const mtc_job_desc *jobs, uint32_t 
   int device = 0, sms = 148;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const uint32_t grid = uint32_t(sms) * shape.ctasPerSm;
-  const uint32_t flagsUnion = reinterpret_cast<const BatchHeader *>(table)->flagsUnion;
+  const BatchHeader *host = reinterpret_cast<const BatchHeader *>(table);
   const BatchHeader *header = (const BatchHeader *)scratch;
-  const bool gpuLayout = (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
-  const BatchKernel kernel = shape.shaped ? shapedNoallocKernel(gpuLayout)
-                             : gpuLayout  ? k_batch_noalloc<true, kPixelThreads, 1>
-                                          : k_batch_noalloc<false, kPixelThreads, 1>;
-  kernel<<<grid, shape.blockThreads, rayColumnBytes(shape.blockThreads), cs>>>(header, queue, counters, shape.grain,
-                                                                               status_out);
+  const BatchGrid grid = batchGrid(shape, host->totalItems, uint32_t(sms));
+  const bool gpuLayout = (host->flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  const BatchKernel kernel = grid.few       ? noallocKernel256(gpuLayout)
+                             : shape.shaped ? shapedNoallocKernel(gpuLayout)
+                             : gpuLayout    ? k_batch_noalloc<true, kPixelThreads, 1>
+                                            : k_batch_noalloc<false, kPixelThreads, 1>;
+  kernel<<<grid.blocks, grid.threads, rayColumnBytes(grid.threads), cs>>>(header, queue, counters, shape.grain,
+                                                                          status_out);
   e = cudaGetLastError();
   return e == cudaSuccess ? MT_OK : MT_ERROR;
 }

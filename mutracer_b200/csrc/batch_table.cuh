@@ -121,6 +121,18 @@ constexpr uint32_t kPixelThreads = 1024;
 // and 7.4 (free-running warps with one thread per pixel: 227 and 8.5).
 constexpr uint32_t kShapedThreads = 128, kShapedBlocks = 4;
 
+// Small images: up to 256 pixels an SM go to 8 warps of one block, a few lanes
+// each.  Few lanes mean little divergence (61x47 pixels, ms with 8 warps of few
+// lanes, 4 of more, full warps in blocks of 1 and of 8: the instanced scene, 4
+// samples, 1.71, 1.92, 2.53 and 3.04; glass, 2 samples, 9.1, 10.4, 12.6 and 14.9;
+// the Cornell box, 4 samples, 1.11, 1.10, 1.17 and 1.28; with one thread per
+// pixel in free-running blocks 4.7, 24.9 and 1.46).  Up to kAlonePixels an SM,
+// each pixel gets a block of one warp and waits for no other, which pays where
+// paths diverge most (24x24 pixels, alone and four to a block: glass 9.7 and
+// 10.6 ms, the instanced scene 1.12 and 1.03, the Cornell box 1.29 and 0.88;
+// free-running threads 43, 4.4 and 1.37).
+constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
+
 struct BatchShape {
   uint32_t blockThreads, tileW, tileH, ctasPerSm, grain;
   bool shaped;  // block size given: kShapedThreads at most
@@ -151,6 +163,27 @@ inline bool batchShape(const mtc_batch_config *c, BatchShape &out) {
     out.grain = c->items_per_fetch;
   }
   return true;
+}
+
+// The grid of a batched launch over `totalItems` work items.  Tables of few
+// pixels run like small images: the grid's blocks share them out (TableClaims),
+// in blocks of kSpreadWarps at 255 registers.  Full warps of blocks of 1,024, on
+// the few SMs whose warps came first, were slower than free-running warps on the
+// Cornell box (61x47 pixels, one sample, free-running / in blocks of 1,024 / so:
+// 0.65, 0.79, 0.44 ms; of the instanced scene 1.71, 1.77, 0.88; 17x13 pixels,
+// three images, 0.57, 0.66, 0.40).  A captured launch may run other tables later:
+// it keeps the blocks of 1,024 and spreads over some of their warps (0.56 ms for
+// the first of these).
+struct BatchGrid {
+  uint32_t blocks, threads;
+  bool few;
+};
+inline BatchGrid batchGrid(const BatchShape &shape, uint32_t totalItems, uint32_t sms) {
+  const uint64_t pixels = uint64_t(totalItems) * 32u, perSm = (pixels + sms - 1u) / sms;
+  if (shape.shaped || shape.ctasPerSm != 1u || perSm > kSpreadWarps * 32u || pixels == 0u)
+    return BatchGrid{sms * shape.ctasPerSm, shape.blockThreads, false};
+  if (perSm <= kAlonePixels) return BatchGrid{uint32_t(pixels), 32u, true};
+  return BatchGrid{sms, kSpreadWarps * 32u, true};
 }
 
 // Writes the header and `job_count` entries of a job table to host memory
@@ -184,10 +217,12 @@ inline mt_status writeBatchTable(const mtc_job_desc *jobs, uint32_t job_count, c
 
 // The pixels of a job table, claimed by the lanes of a persistent grid.
 // queue[0] is the next work item; items are warp tiles (tileW x 32/tileW
-// pixels) laid out job after job (JobData.firstItem / .items).  A warp takes
-// `grain` consecutive items per atomic and hands their pixels to its lanes as
-// they ask.  A warp is done when the counter passes the item total; its fetch
-// bound only guards against a corrupted table, and running out of it sets
+// pixels) laid out job after job (JobData.firstItem / .items), or, where the
+// table has few for the grid (kSpread), slices of them: then some warps of a
+// block ask, with as many lanes as a slice has pixels.  A warp takes `grain`
+// consecutive items per atomic and hands their pixels to its lanes as they ask.
+// A warp is done when the counter passes the item total; its fetch bound only
+// guards against a corrupted table, and running out of it sets
 // kBatchStatusGuardExhausted in `status` (when given).
 struct TableClaims {
   const BatchHeader *header;
@@ -195,16 +230,24 @@ struct TableClaims {
   uint32_t *queue;
   uint32_t *status;
   uint32_t grain;
-  uint64_t cursor = 0, end = 0;  // units (pixels of the tiles taken) left
+  uint32_t slice = 32u;          // pixels of an item, a power of two
+  uint64_t cursor = 0, end = 0;  // units (pixels of the items taken) left
   uint32_t fetches = 0;
   bool exhausted = false;
 
-  MTD TableClaims(const BatchHeader *h, uint32_t *q, uint32_t *st, uint32_t g)
+  MTD TableClaims(const BatchHeader *h, uint32_t *q, uint32_t *st, uint32_t g, bool spread)
       : header(h), jobs(reinterpret_cast<const JobData *>(reinterpret_cast<const char *>(h) + kBatchTableOffset)),
-        queue(q), status(st), grain(g) {}
+        queue(q), status(st), grain(g) {
+    const uint64_t perBlock = (uint64_t(h->totalItems) * 32u + gridDim.x - 1u) / gridDim.x;
+    if (!spread || perBlock > kSpreadWarps * 32u) return;
+    const uint32_t warps = min(min(kSpreadWarps, blockDim.x / 32u), uint32_t(perBlock));
+    exhausted = threadIdx.x / 32u >= warps;
+    while (slice / 2u * warps >= perBlock && slice > 1u) slice /= 2u;
+  }
 
   MTD void next(bool wants, const JobData *&job, uint32_t &x, uint32_t &y, uint32_t &samples) {
-    const uint32_t lane = threadIdx.x & 31u, total = header->totalItems, tileW = header->tileW;
+    const uint32_t lane = threadIdx.x & 31u, total = header->totalItems * (32u / slice), tileW = header->tileW;
+    wants = wants && lane < slice;
     unsigned asking = __ballot_sync(0xffffffffu, wants);
     while (asking && !exhausted) {
       if (cursor == end) {
@@ -216,8 +259,8 @@ struct TableClaims {
           exhausted = true;
           break;
         }
-        cursor = uint64_t(first) * 32u;
-        end = uint64_t(min(first + grain, total)) * 32u;
+        cursor = uint64_t(first) * slice;
+        end = uint64_t(min(first + grain, total)) * slice;
       }
       const uint64_t u = cursor + __popc(asking & ((1u << lane) - 1u));
       cursor = min(end, cursor + uint64_t(__popc(asking)));
@@ -246,10 +289,10 @@ struct TableClaims {
 };
 
 // The persistent work loop of the batched kernels.
-template <bool kGpuLayout>
+template <bool kGpuLayout, bool kSpread>
 __device__ __forceinline__ void batchWorkLoop(const BatchHeader *__restrict__ header, uint32_t *queue, uint32_t grain,
                                               uint32_t *status, Counters &cnt, uint32_t &paths) {
-  TableClaims claims(header, queue, status, grain);
+  TableClaims claims(header, queue, status, grain, kSpread);
   tracePixels<kGpuLayout>(claims, cnt, paths);
 }
 

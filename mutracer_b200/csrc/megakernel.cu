@@ -24,18 +24,6 @@ using namespace mt;
 
 namespace {
 
-// Small images: up to 256 pixels an SM go to 8 warps of one block, a few lanes
-// each.  Few lanes mean little divergence (61x47 pixels, ms with 8 warps of few
-// lanes, 4 of more, full warps in blocks of 1 and of 8: the instanced scene, 4
-// samples, 1.71, 1.92, 2.53 and 3.04; glass, 2 samples, 9.1, 10.4, 12.6 and 14.9;
-// the Cornell box, 4 samples, 1.11, 1.10, 1.17 and 1.28; with one thread per
-// pixel in free-running blocks 4.7, 24.9 and 1.46).  Up to kAlonePixels an SM,
-// each pixel gets a block of one warp and waits for no other, which pays where
-// paths diverge most (24x24 pixels, alone and four to a block: glass 9.7 and
-// 10.6 ms, the instanced scene 1.12 and 1.03, the Cornell box 1.29 and 0.88;
-// free-running threads 43, 4.4 and 1.37).
-constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
-
 // Large images: a block holds its SM until it ends, and a stream of higher
 // priority is let in only then, so a block gets about kBlockPixels pixels (a pick
 // during a 1080p render of the instanced scene, 4 samples, 91 ms, waits 20 ms at
@@ -430,16 +418,21 @@ mt_status launchBatch(const void *table, uint32_t capacity, const BatchShape &sh
   e = cudaGetDevice(&device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return cudaStatus(e);
-  // A full persistent grid: the item total is only known on the device.
-  uint32_t grid = uint32_t(sms) * shape.ctasPerSm;
-  // The host copy of the header decides the BLAS-layout specialisation.
-  uint32_t flagsUnion = static_cast<const BatchHeader *>(table)->flagsUnion;
-  const bool gpuLayout = (flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
-  const BatchKernel kernel = shape.shaped ? shapedBatchKernel(gpuLayout)
-                             : gpuLayout  ? k_batch<true, kPixelThreads, 1>
-                                          : k_batch<false, kPixelThreads, 1>;
-  kernel<<<grid, shape.blockThreads, rayColumnBytes(shape.blockThreads), st>>>((const BatchHeader *)scratch, queue,
-                                                                               counters, shape.grain, status);
+  // The host copy of the header decides the BLAS-layout specialisation and,
+  // unless a graph is being captured, which may run with other tables, the grid.
+  const BatchHeader *host = static_cast<const BatchHeader *>(table);
+  const bool gpuLayout = (host->flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  e = cudaStreamIsCapturing(st, &capture);
+  if (e != cudaSuccess) return cudaStatus(e);
+  const bool fixed = capture == cudaStreamCaptureStatusNone;
+  const BatchGrid grid = batchGrid(shape, fixed ? host->totalItems : UINT32_MAX, uint32_t(sms));
+  const BatchKernel kernel = grid.few       ? batchKernel256(gpuLayout)
+                             : shape.shaped ? shapedBatchKernel(gpuLayout)
+                             : gpuLayout    ? k_batch<true, kPixelThreads, 1>
+                                            : k_batch<false, kPixelThreads, 1>;
+  kernel<<<grid.blocks, grid.threads, rayColumnBytes(grid.threads), st>>>((const BatchHeader *)scratch, queue, counters,
+                                                                          shape.grain, status);
   return cudaStatus(cudaGetLastError());
 }
 

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
     k_batch(const BatchHeader *header, uint32_t *queue, mtc_counters *counters, uint32_t grain, uint32_t *status) {
   Counters cnt;
   uint32_t paths = 0;
-  batchWorkLoop<kGpuLayout>(header, queue, grain, status, cnt, paths);
+  batchWorkLoop<kGpuLayout, kThreads != kShapedThreads>(header, queue, grain, status, cnt, paths);
   flushCounters(cnt, paths, counters);
 }
 
@@ -117,12 +117,15 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
                     uint32_t *status) {
   Counters cnt;
   uint32_t paths = 0;
-  batchWorkLoop<kGpuLayout>(header, queue, grain, status, cnt, paths);
+  batchWorkLoop<kGpuLayout, kThreads != kShapedThreads>(header, queue, grain, status, cnt, paths);
   addCounters(cnt, paths, counters);
 }
 
 // The kernels for blocks of a size that the host gave (kShapedThreads at most).
 BatchKernel shapedBatchKernel(bool gpuLayout);
 BatchKernel shapedNoallocKernel(bool gpuLayout);
+// The kernels for blocks of up to 256 threads (BatchGrid.few).
+BatchKernel batchKernel256(bool gpuLayout);
+BatchKernel noallocKernel256(bool gpuLayout);
 
 }  // namespace mt

@@ -111,3 +111,44 @@ def test_plain_kernels_of_every_block_size(cuda, size, layout):
     torch.cuda.synchronize()
     assert (plain.acc.normal[:, 3] == 2).all()
     assert _same(plain.acc, job.acc)
+
+
+@pytest.mark.parametrize("layout", [0, 2])
+@pytest.mark.parametrize("sizes", [[(1, 1)], [(7, 5), (3, 9)], [(24, 24)], [(37, 29)] * 3, [(61, 47)],
+                                   [(199, 150), (64, 33)], [(300, 130)]])
+def test_tables_of_few_pixels(cuda, sizes, layout):
+    """One pixel a block, slices of every size, and the first table that is not
+    spread: each image that of its own launch, with any number of items a fetch,
+    in a captured launch that then runs another table, and over fixed scratch."""
+    import torch
+    jobs, want = [], []
+    for k, (w, h) in enumerate(sizes):
+        host = scene.SceneHost("instanced_spheres", w, h, 3 + k, (24, 3, 4, 64, 2))
+        if layout:
+            host.set_blas_layout(layout)
+        dev = scene.DeviceScene(host, cuda)
+        jobs.append(batch.RenderJob(dev, 2 + k, device=cuda))
+        want.append(batch.RenderJob(dev, 2 + k, device=cuda))
+        want[-1].render_alone()
+
+    def check(run):
+        for j in jobs:
+            j.acc.zero_()
+        torch.cuda.synchronize()
+        run()
+        torch.cuda.synchronize()
+        for a, b in zip(want, jobs):
+            assert (a.acc.normal[:, 3] == a.spp).all() and _same(a.acc, b.acc)
+
+    for cfg in ((0, 0, 0, 0), (0, 2, 0, 16), (0, 32, 2, 3)):
+        b = batch.Batch(len(jobs), abi.BatchConfig.make(*cfg), cuda)
+        b.set_jobs(jobs)
+        check(b.launch)
+    b = batch.Batch(len(jobs), device=cuda)
+    b.set_jobs(jobs[:1])
+    b.capture()
+    b.set_jobs(jobs)
+    check(b.replay)
+    descs = (abi.JobDesc * len(jobs))(*[j.desc(j.spp) for j in jobs])
+    check(lambda: abi.check(abi.lib().mtc_trace_batch_noalloc(
+        descs, len(jobs), None, None, None, C.c_void_p(torch.cuda.current_stream().cuda_stream))))
