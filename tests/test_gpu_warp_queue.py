@@ -144,3 +144,20 @@ def test_build_and_refit_at_run_edges(cuda, side):
         assert buf.cpu().numpy().tobytes() == boxes.tobytes()
         # sums of n positive float64 terms in two orders: n rounding steps each
         assert abs(area - host_area) <= 2 * len(want) * np.finfo(np.float64).eps * host_area
+
+
+def test_refit_area_in_one_launch_and_in_two(cuda):
+    """Buffers of up to 591 vec4 hold no more nodes than the area sum has runs: it
+    is one launch there, two from 592 on, and the same bits."""
+    import torch
+    pos, idx = blas.terrain_mesh(2, 20, seed=4)
+    want, _ = blas.host_build(pos, idx)
+    moved = torch.from_numpy((pos * np.float32(1.5)).astype(np.float32)).to(cuda)
+    boxes, host_area = blas.host_refit(want, moved.cpu().numpy())
+    areas = []
+    for vec4 in (len(want) // 4, 588, 589, 590, 591, 592, 593, 700):
+        buf = torch.zeros(vec4 * 4, dtype=torch.float32, device=cuda)
+        buf[:len(want)] = torch.from_numpy(want.view(np.float32)).to(cuda)
+        areas.append(blas.BlasRefit(buf).refit(moved).item())
+        assert buf[:len(want)].cpu().numpy().tobytes() == boxes.tobytes()
+    assert len(set(areas)) == 1 and abs(areas[0] - host_area) <= 2 * len(want) * np.finfo(np.float64).eps * host_area
