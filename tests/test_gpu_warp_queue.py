@@ -161,3 +161,76 @@ def test_refit_area_in_one_launch_and_in_two(cuda):
         areas.append(blas.BlasRefit(buf).refit(moved).item())
         assert buf[:len(want)].cpu().numpy().tobytes() == boxes.tobytes()
     assert len(set(areas)) == 1 and abs(areas[0] - host_area) <= 2 * len(want) * np.finfo(np.float64).eps * host_area
+
+
+def _records(words, ints, node, rel):
+    """The leaf records below `node`, and the first vec4 past the subtree
+    (right pointers are relative to `rel`)."""
+    ptr = int(ints[node, 3])
+    if ptr < 0:
+        return [words[node + 2 + k].copy() for k in range(-ptr)], node + 2 - ptr
+    left, _ = _records(words, ints, node + 2, rel)
+    right, end = _records(words, ints, rel + ptr, rel)
+    return left + right, end
+
+
+def _chain(words, ints, node, rel, records, depth):
+    """Overwrites the subtree at `node` with a chain: every right child a leaf
+    of one record, every left child the rest, the last leaf holding what is
+    left; all boxes those of the root, so that a ray takes all left children
+    with every right one on the stack."""
+    lo, hi = words[node].copy(), words[node + 1].copy()
+    inner = [node + 2 * k for k in range(depth + 1)]
+    at = inner[-1]
+    for k in range(depth, -1, -1):  # the last left child, then right children from the deepest
+        rest = records[depth:] if k == depth else records[k:k + 1]
+        words[at], words[at + 1] = lo, hi
+        ints[at, 3] = -len(rest)
+        words[at + 2:at + 2 + len(rest)] = rest
+        if k < depth:
+            words[inner[k]], words[inner[k] + 1] = lo, hi
+            ints[inner[k], 3] = at - rel
+        at += 2 + len(rest)
+    return at
+
+
+@pytest.mark.parametrize("level", ["tlas", "blas"])
+@pytest.mark.parametrize("depth", [62, 63, 64, 90])
+def test_trees_deeper_than_the_traversal_stack(cuda, level, depth):
+    """Chains that fill the 64 entries of a level's stack: the nearer child of a
+    node that finds one entry left is dropped, as in the reference, and what is
+    below it never hit.  Bit-exact against the oracle in every engine."""
+    import torch
+    host = scene.SceneHost("instanced_spheres", 40, 24, 3, (400, 1, 6, 64, 2))
+    rays = oracle_lib.seeded_rays(host, 3000, seed=depth)
+    whole = oracle_lib.first_hits(host, rays)
+    words = host.bvh.reshape(-1, 4)
+    ints = words.view(np.int32)
+    if level == "tlas":
+        root, rel = 0, 0
+    else:
+        base = host.uniform.blas_offset
+        roots = {(base + int(e[1]), base + int(host.instances.view(np.int32)[int(e[0]) * 40] & 0x3fffffff))
+                 for e in (r.view(np.int32) for r in _records(words, ints, 0, 0)[0])}
+        root, rel = max(roots, key=lambda r: len(_records(words, ints, *r)[0]))  # the spheres' mesh
+    records, end = _records(words, ints, root, rel)
+    assert len(records) > depth + 20
+    assert _chain(words, ints, root, rel, records, depth) <= end
+    want = oracle_lib.first_hits(host, rays)
+    got = trace.query_first_hit(scene.DeviceScene(host, cuda), torch.from_numpy(rays).to(cuda)).cpu().numpy()
+    same, tie = _hits_equal(got, want)
+    assert (same | tie).all()
+    fewer = int(want.view(np.int32).reshape(len(rays), -1)[:, 0].sum()) < int(
+        whole.view(np.int32).reshape(len(rays), -1)[:, 0].sum())
+    assert fewer == (depth >= 64), "the limit is met at the depth it should be"
+    dev = scene.DeviceScene(host, cuda)
+    plain, one, job = (batch.RenderJob(dev, 2, device=cuda) for _ in range(3))
+    plain.render_alone()
+    b = batch.Batch(1, device=cuda)
+    b.set_jobs([one])
+    b.launch()
+    sb = batch.StreamBatch(1, stream_config=abi.StreamConfig.make(slots=1024), device=cuda)
+    sb.set_jobs([job])
+    sb.run()
+    torch.cuda.synchronize()
+    assert _same(plain.acc, one.acc) and _same(plain.acc, job.acc)
