@@ -126,12 +126,15 @@ constexpr uint32_t kShapedThreads = 128, kShapedBlocks = 4;
 // lanes, 4 of more, full warps in blocks of 1 and of 8: the instanced scene, 4
 // samples, 1.71, 1.92, 2.53 and 3.04; glass, 2 samples, 9.1, 10.4, 12.6 and 14.9;
 // the Cornell box, 4 samples, 1.11, 1.10, 1.17 and 1.28; with one thread per
-// pixel in free-running blocks 4.7, 24.9 and 1.46).  Up to kAlonePixels an SM,
-// each pixel gets a block of one warp and waits for no other, which pays where
-// paths diverge most (24x24 pixels, alone and four to a block: glass 9.7 and
-// 10.6 ms, the instanced scene 1.12 and 1.03, the Cornell box 1.29 and 0.88;
-// free-running threads 43, 4.4 and 1.37).
-constexpr uint32_t kSpreadWarps = 8, kAlonePixels = 4;
+// pixel in free-running blocks 4.7, 24.9 and 1.46).  That is a choice for the
+// latency of one render: it takes some of every SM, and several at a time hold
+// one another up where paths hardly diverge (61x47 Cornell boxes on 1, 2, 4 and
+// 8 streams 0.42, 0.65, 1.08 and 1.95 ms, free-running 0.56, 0.59, 0.68 and
+// 1.09; the instanced scene 0.72, 0.93, 1.43 and 2.48 against 1.69, 1.69, 1.76
+// and 2.21; glass 5.3, 5.5, 9.2 and 15.2 against 14 to 20).  64 or 128 registers
+// hardly help those and cost one render 15 to 35 %; a block of one warp for each
+// pixel of the smallest images made eight of 24x24 take 1.63 ms, not 1.20.
+constexpr uint32_t kSpreadWarps = 8;
 
 struct BatchShape {
   uint32_t blockThreads, tileW, tileH, ctasPerSm, grain;
@@ -182,8 +185,7 @@ inline BatchGrid batchGrid(const BatchShape &shape, uint32_t totalItems, uint32_
   const uint64_t pixels = uint64_t(totalItems) * 32u, perSm = (pixels + sms - 1u) / sms;
   if (shape.shaped || shape.ctasPerSm != 1u || perSm > kSpreadWarps * 32u || pixels == 0u)
     return BatchGrid{sms * shape.ctasPerSm, shape.blockThreads, false};
-  if (perSm <= kAlonePixels) return BatchGrid{uint32_t(pixels), 32u, true};
-  return BatchGrid{sms, kSpreadWarps * 32u, true};
+  return BatchGrid{sms, uint32_t(perSm < kSpreadWarps ? perSm : kSpreadWarps) * 32u, true};
 }
 
 // Writes the header and `job_count` entries of a job table to host memory

@@ -316,15 +316,11 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
   // One block an SM, of as many warps as it has pixels for.
   const uint64_t units = uint64_t((J.width + 7) / 8) * ((J.height + 3) / 4) * 32u;
   const uint64_t perSm = std::max<uint64_t>(1, (units + uint64_t(sms) - 1) / uint64_t(sms));
-  uint32_t warps = uint32_t(std::min<uint64_t>(
+  const uint32_t warps = uint32_t(std::min<uint64_t>(
       kPixelThreads / 32, perSm <= kSpreadWarps * 32u ? std::min<uint64_t>(kSpreadWarps, perSm) : (perSm + 31) / 32));
   ImageSplit split;
   split.lanes = uint32_t(std::min<uint64_t>(32, (perSm + warps - 1) / warps));
   uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms), units)));
-  if (perSm <= kAlonePixels) {
-    warps = split.lanes = 1;
-    grid = uint32_t(std::max<uint64_t>(1, units));
-  }
   const uint32_t turns = uint32_t(std::max<uint64_t>(1, perSm / kBlockPixels));
   split.run = turns == 1 && perSm > kPixelThreads ? kRunPixels : warps * split.lanes;
   grid *= turns;
