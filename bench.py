@@ -164,13 +164,13 @@ def oracle_traffic(host, rows=8, spp=2):
 
 
 # DRAM bytes (read + write) measured by ncu, per unit of work: the plain
-# megakernel per path sample, the wavefront kernels per queued ray or
-# finished path (small-case captures; the wavefront's normalised by exact
-# queue lengths), scaled by the units this step processed.
+# megakernel per path sample, the wavefront kernels per queued ray, k_wf_finish
+# per path that ended (most end in k_wf_shade); small-case captures normalised
+# by exact counts, scaled by the units this step processed.
 MEGAKERNEL_TRAFFIC = ("k_trace_instanced_spheres_960x540_4spp.md", "dram_bytes_per_path:")
 WAVEFRONT_TRAFFIC = ("wavefront_dram_per_kernel_instanced_spheres_960x540_4spp.md",
                      ("dram_bytes_per_extension_ray:", "dram_bytes_per_shaded_ray:", "dram_bytes_per_shadow_ray:",
-                      "dram_bytes_per_finished_path:"))
+                      "dram_bytes_per_ended_path:"))
 
 
 def _profile_values(name, keys):
@@ -303,10 +303,10 @@ def queue_trace(sb, counters, slots, iterations):
     repeated from zeroed accumulation (a pixel's sample index is its
     accumulated count), stopped by its iteration limit after 1, 2, ...
     `iterations` iterations, and the counter totals are differenced.  For an RGB
-    scene every queued extension ray is traced and every finished slot ends a
-    path, so the three counts are the queue lengths k_wf_extend (and
-    k_wf_shade), k_wf_shadow and k_wf_finish see in that iteration; they
-    normalise single-launch profiler captures to bytes per ray."""
+    scene every queued extension ray is traced, so the first two counts are the
+    queue lengths k_wf_extend (and k_wf_shade) and k_wf_shadow see in that
+    iteration, and the third is the paths that ended in it, in k_wf_shade or
+    k_wf_finish; they normalise single-launch profiler captures."""
     import torch
     from mutracer_b200 import abi
     rows, last = [], [0, 0, 0]
@@ -443,7 +443,7 @@ def run_b200(args):
                               "peak_source": peak_kind,
                               "bytes_per_path": round(bpp, 1),
                               "kernel": "k_trace (one launch per step)" if args.form == "megakernel" else
-                              "all wavefront kernels of the step (k_wf_extend the largest, ~44 %)",
+                              "all wavefront kernels of the step (k_wf_extend the largest)",
                               "traffic_source": source}
     except Exception as exc:  # the oracle library may be absent on a box
         result["roofline"] = {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None,
