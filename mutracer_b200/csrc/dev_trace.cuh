@@ -343,7 +343,8 @@ struct TraversalHit {
 // to enter, or the triangles of a BLAS leaf; advance() runs one of these at a
 // time for all lanes of the warp that are at it.  A lane that waits only
 // waits: each ray's visit order, box tests, `>` tie rule and self-hit and
-// backface rules are those of traverse(), so the hits are bit-identical to it.
+// backface rules are those of the reference's loop, so the hits are bit-identical
+// to its.
 //
 // What bounds it is issue slots at few active lanes.  With every lane taking
 // whatever step came next, an iteration ran the node code for ~20 lanes, the

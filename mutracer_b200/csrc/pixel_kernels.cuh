@@ -74,10 +74,10 @@ struct ImageClaims {
 
 // The plain megakernel.  Bound by instruction fetch and by the latency of its
 // spilled state; with the 32 warps of an SM's block in step 4 samples of the
-// 4M-triangle instanced scene at 960x540 take 29.2 ms (64 free-running warps
-// an SM with one thread per pixel: 67.2), 8 of the Cornell box at 512x512 13.8
-// (29.6), one of the glass scene at 640x360 24.0 (85.2), one of a 256x256
-// Cornell box 1.1 (2.5).  Free-running warps that trace and shade together,
+// 4M-triangle instanced scene at 960x540 take 29.5 ms (64 free-running warps
+// an SM with one thread per pixel: 67.2), 8 of the Cornell box at 512x512 12.8
+// (29.6), one of the glass scene at 640x360 20.4 (85.2), one of a 256x256
+// Cornell box 0.78 (1.9).  Free-running warps that trace and shade together,
 // or that shade once 8, 12 or 20 lanes wait, are slower than one thread per
 // pixel: it is the fetches shared by the block that pay.
 template <bool kGpuLayout, uint32_t kThreads>

@@ -256,12 +256,9 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_seed(StreamView v, uint32
   flush(v, 0, 0, 0);
 }
 
-// Closest hits of the queued extension rays.  Persistent: a lane whose ray
-// has finished takes the next queued ray at once, so a warp is not held by
-// its slowest ray (traversal lengths differ by an order of magnitude here).
 // Resident CTAs per SM of the traversal kernels: the closest-hit kernel at
 // 5 holds its traversal state in 87 registers and the shadow kernel at 6 in
-// 78, without spilling (6 and 7 CTAs: within 1 % on the 1080p instanced
+// 76 (80 with coverage), without spilling (6 and 7 CTAs: within 1 % on the 1080p instanced
 // scene, 4 % slower on the glass scene).
 #ifndef MT_EXTEND_MIN_BLOCKS
 #define MT_EXTEND_MIN_BLOCKS 5
@@ -269,9 +266,11 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_seed(StreamView v, uint32
 #ifndef MT_SHADOW_MIN_BLOCKS
 #define MT_SHADOW_MIN_BLOCKS 6
 #endif
-// Drains a queue of `count` rays behind the counter `next` with every warp of
-// the grid.  Where there are fewer rays than lanes, the batches shrink so
-// that every warp gets some.
+// Drains the `count` rays of a source's queue with every warp of the grid.  A
+// lane whose ray has finished takes a next one, so a warp is not held by its
+// slowest ray (traversal lengths differ by an order of magnitude here).  Where
+// there are fewer rays than lanes, the batches shrink so that every warp gets
+// some.
 template <bool shadow, bool kGpuLayout, bool kAlpha, class Source>
 MTD void drainQueue(const StreamView &v, Source &src, uint32_t count) {
   __shared__ WarpRays rays[kStreamThreads / 32];
@@ -308,9 +307,8 @@ struct ExtendSource {
     const JobData &J = v.jobs[sl.job];
     q.payload = s;
     q.scene = sl.job;
-    // traceExtension: an empty scene is a miss without a traversal, and a
-    // spectral wavelength path restarting at the shared primary vertex
-    // traces nothing.
+    // An empty scene is a miss without a traversal, and a spectral wavelength
+    // path restarting at the shared primary vertex traces nothing.
     if (J.u.is_empty > 0 || (isSpectral(J) && reusesPrimary(J, sl.ps, v.spectral[s].primaryReady)) ||
         (alphaSplit(J) && v.spectral[s].frontPending)) {
       missed(q);
@@ -400,13 +398,16 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_sort_rays(StreamView v) {
 }
 
 // A long shading queue starts with the costly classes, so that misses and
-// plain diffuse hits are left for its tail (119.5 against 124.3 ms, 8 samples
-// of the 1080p instanced scene, 2M rays); one of a few chunks a block keeps
-// the ascending order (30.9 against 32.4 ms, Cornell box, 262k rays).
+// plain diffuse hits are left for its tail; a shorter one keeps the ascending
+// order.  ms always costly first / never / so, by the image that fills the
+// queue: instanced scene 1920x1080 28.8 / 30.5 / 28.9, 1024x1024 21.0 / 21.8 /
+// 21.1, 725x725 26.3 / 27.7 / 27.3, 512x512 19.7 / 20.0 / 20.1; Cornell box
+// 1024x1024 13.3 / 13.0 / 13.3, 725x725 14.5 / 14.1 / 14.4, 512x512 8.5 / 8.1 /
+// 8.1; glass 1024x1024 73.3 / 71.6 / 71.7, 725x725 91.8 / 90.9 / 90.7.
 constexpr uint32_t kCostlyFirstRays = 1u << 19;
 
 // Orders the extension queue by material class (counting sort on the keys
-// counted by k_wf_extend), so that the warps shading at any one time run the
+// counted by k_wf_classify), so that the warps shading at any one time run the
 // same BSDF code.  The order of slots inside a class is arbitrary; it cannot
 // change any result, since slots never share state.
 __global__ void __launch_bounds__(kStreamThreads) k_wf_regroup(StreamView v) {
@@ -443,13 +444,12 @@ __global__ void __launch_bounds__(kStreamThreads) k_wf_regroup(StreamView v) {
 // and over the code fetched it apart (28 of 55 stall cycles per issue waited
 // for instructions).  So the class-ordered queue is handed out in chunks from
 // one counter, which keeps the SM's blocks in one class at a time, and the
-// four warps of a block start each chunk together (10.5 of 26 stall cycles; one
-// block of 512 threads an SM in step: 3 of 16, 2.61 -> 1.89 ms for 1.45M rays).
-// With fetches shared, more registers and fewer
-// warps win: 4 blocks at 128 registers against 8 at 64 (124.3 and 125.3 ms,
-// 8 samples of the 1080p instanced scene; 30.9 and 32.8 ms, 16 samples of the
-// Cornell box).  Blocks of 256 and 512 threads: 2 % faster on the first, 2 to
-// 8 % slower on the second, which has only 3.5 chunks a block.
+// four warps of a block start each chunk together (10.5 of 26 stall cycles; 1.45M
+// rays 2.56 -> 2.40 ms, with most of k_wf_finish's work).  With fetches shared,
+// more registers and fewer warps win: 4 blocks at 128 registers against 8 at 64
+// (124.3 and 125.3 ms, 8 samples of the 1080p instanced scene; 30.9 and 32.8 ms,
+// 16 samples of the Cornell box).  Blocks of 256 and 512 threads: 2 % faster on
+// the first, 2 to 8 % slower on the second, which has only 3.5 chunks a block.
 constexpr int kShadeThreads = 128;
 #ifndef MT_SHADE_MIN_BLOCKS
 #define MT_SHADE_MIN_BLOCKS 4
@@ -520,10 +520,10 @@ __global__ void __launch_bounds__(kShadeThreads, MT_SHADE_MIN_BLOCKS)
   flush(v, 0, 0, paths);
 }
 
-// NEE visibility of the queued shadow rays (intersectSceneShadow).  An
+// NEE visibility of the queued shadow rays.  An
 // occluded query is marked in its slot, a store that nothing waits for; the
 // kernel that reads the slot next adds the contributions of the others
-// (addUnoccluded, the sum of resolveShadow).
+// (addUnoccluded).
 struct ShadowSource {
   const StreamView &v;
   uint32_t rays;
