@@ -33,13 +33,17 @@ namespace {
 // 45.7 ms for 2 samples of that scene, 16.0 against 15.2 of the Cornell box;
 // blocks of 3,072 pixels 49.7 and 17.6, of 2,048 46.7 and 18.4.
 constexpr uint64_t kBlockPixels = 4096;
-// A single block an SM takes turns at runs of kRunPixels pixels, which leaves no
-// two blocks more than one run apart (runs of 1,024: up to 1,024 pixels apart;
-// 801x601, 2 samples, Cornell box 5.20 against 5.79 ms, instanced scene 8.55 and
-// 9.26; one sample of 401x378 1.47 and 1.68; runs of 256 and 32 within 3 % of
-// 64).  With blocks to follow, runs of a pixel a lane keep neighbours together:
-// 46.1 against 49.5 ms with runs of 128 in the 1080p render above.
-constexpr uint32_t kRunPixels = 64;
+// A single block an SM takes turns at runs of the image.  Long runs keep the
+// block at one place, whose paths share code and length; short ones deal the work
+// evenly.  kRunPixels, or half of that where it would leave the fullest block more
+// than 1/12 above the mean (ms at 256 / 512 / 1,024 pixels: instanced scene 801x601
+// 13.7 / 14.1 / 16.4, 640x360 14.8 / 14.7 / 19.3, 1280x720 22.6 / 21.2 / 21.6; glass
+// 801x601 26.7 / 28.7 / 29.4; Cornell box 801x601 5.3 / 5.4 / 5.7, 512x512 16.5 /
+// 17.7 / 17.4).  Scenes with coverage, whose shadow rays differ most from place to
+// place, keep runs of a pixel a lane (a room 801x601 13.4 / 12.6 / 12.0, 512x512
+// 8.7 / 7.8 / 7.8; 15.0 and 9.8 at 64).  So do images with blocks to follow: 46.1
+// against 49.5 ms with runs of 128 in the 1080p render above.
+constexpr uint32_t kRunPixels = 512;
 
 __global__ void k_sample_maps(const __grid_constant__ DevScene s, const int32_t *indices, const float2 *uvs,
                               uint32_t count, float4 *out) {
@@ -323,7 +327,12 @@ mt_status mtc_trace_samples(const mtc_scene_view *scene, const mtc_camera_unifor
   split.lanes = uint32_t(std::min<uint64_t>(32, (perSm + warps - 1) / warps));
   uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms), units)));
   const uint32_t turns = uint32_t(std::max<uint64_t>(1, perSm / kBlockPixels));
-  split.run = turns == 1 && perSm > kPixelThreads ? kRunPixels : warps * split.lanes;
+  split.run = warps * split.lanes;
+  if (turns == 1 && perSm > kPixelThreads && !(scene->flags & MTC_SCENE_HAS_ALPHA)) {
+    const uint64_t runs = (units + kRunPixels - 1) / kRunPixels;
+    const uint64_t fullest = (runs + uint64_t(sms) - 1) / uint64_t(sms) * kRunPixels;
+    split.run = fullest * 12 <= perSm * 13 ? kRunPixels : kRunPixels / 2;
+  }
   grid *= turns;
   // The most registers that blocks of so many warps leave room for: 24x24 pixels
   // of the Cornell box, 4 samples, 1.29 ms (1.57 at 64 registers); 256x256, one
