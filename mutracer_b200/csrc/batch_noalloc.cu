@@ -130,6 +130,7 @@ extern "C" mt_status mtc_trace_batch_noalloc(const mtc_job_desc *jobs, uint32_t 
   const BatchGrid grid = batchGrid(shape, host->totalItems, uint32_t(sms));
   const bool gpuLayout = (host->flagsUnion & MTC_SCENE_BLAS_GPU_LAYOUT) != 0u;
   const BatchKernel kernel = grid.few       ? noallocKernel256(gpuLayout)
+                             : grid.medium  ? noallocKernel512(gpuLayout)
                              : shape.shaped ? shapedNoallocKernel(gpuLayout)
                              : gpuLayout    ? k_batch_noalloc<true, kPixelThreads, 1>
                                             : k_batch_noalloc<false, kPixelThreads, 1>;

@@ -176,16 +176,21 @@ inline bool batchShape(const mtc_batch_config *c, BatchShape &out) {
 // 0.65, 0.79, 0.44 ms; of the instanced scene 1.71, 1.77, 0.88; 17x13 pixels,
 // three images, 0.57, 0.66, 0.40).  A captured launch may run other tables later:
 // it keeps the blocks of 1,024 and spreads over some of their warps (0.56 ms for
-// the first of these).
+// the first of these).  Up to kMediumPixels an SM, 16 warps at 128 registers have
+// a lane for every pixel: 333x217 pixels, in blocks of 1,024 / so, Cornell box
+// 2.50, 1.87 ms; instanced scene 5.03, 3.99; glass 19.9, 16.3; room 4.69, 4.10.
+constexpr uint32_t kMediumPixels = 512;
 struct BatchGrid {
   uint32_t blocks, threads;
-  bool few;
+  bool few;     // blocks of up to 256 threads
+  bool medium;  // of 512
 };
 inline BatchGrid batchGrid(const BatchShape &shape, uint32_t totalItems, uint32_t sms) {
   const uint64_t pixels = uint64_t(totalItems) * 32u, perSm = (pixels + sms - 1u) / sms;
-  if (shape.shaped || shape.ctasPerSm != 1u || perSm > kSpreadWarps * 32u || pixels == 0u)
-    return BatchGrid{sms * shape.ctasPerSm, shape.blockThreads, false};
-  return BatchGrid{sms, uint32_t(perSm < kSpreadWarps ? perSm : kSpreadWarps) * 32u, true};
+  if (shape.shaped || shape.ctasPerSm != 1u || perSm > kMediumPixels || pixels == 0u)
+    return BatchGrid{sms * shape.ctasPerSm, shape.blockThreads, false, false};
+  if (perSm > kSpreadWarps * 32u) return BatchGrid{sms, kMediumPixels, false, true};
+  return BatchGrid{sms, uint32_t(perSm < kSpreadWarps ? perSm : kSpreadWarps) * 32u, true, false};
 }
 
 // Writes the header and `job_count` entries of a job table to host memory

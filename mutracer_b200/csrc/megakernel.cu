@@ -434,6 +434,7 @@ mt_status launchBatch(const void *table, uint32_t capacity, const BatchShape &sh
   const bool fixed = capture == cudaStreamCaptureStatusNone;
   const BatchGrid grid = batchGrid(shape, fixed ? host->totalItems : UINT32_MAX, uint32_t(sms));
   const BatchKernel kernel = grid.few       ? batchKernel256(gpuLayout)
+                             : grid.medium  ? batchKernel512(gpuLayout)
                              : shape.shaped ? shapedBatchKernel(gpuLayout)
                              : gpuLayout    ? k_batch<true, kPixelThreads, 1>
                                             : k_batch<false, kPixelThreads, 1>;

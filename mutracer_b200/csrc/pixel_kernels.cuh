@@ -124,7 +124,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
 // The kernels for blocks of a size that the host gave (kShapedThreads at most).
 BatchKernel shapedBatchKernel(bool gpuLayout);
 BatchKernel shapedNoallocKernel(bool gpuLayout);
-// The kernels for blocks of up to 256 threads (BatchGrid.few).
+// The kernels for blocks of 512 and of up to 256 threads (BatchGrid).
+BatchKernel batchKernel512(bool gpuLayout);
+BatchKernel noallocKernel512(bool gpuLayout);
 BatchKernel batchKernel256(bool gpuLayout);
 BatchKernel noallocKernel256(bool gpuLayout);
 
