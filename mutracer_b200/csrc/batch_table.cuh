@@ -246,9 +246,14 @@ struct TableClaims {
       : header(h), jobs(reinterpret_cast<const JobData *>(reinterpret_cast<const char *>(h) + kBatchTableOffset)),
         queue(q), status(st), grain(g) {
     const uint64_t perBlock = (uint64_t(h->totalItems) * 32u + gridDim.x - 1u) / gridDim.x;
-    if (!spread || perBlock > kSpreadWarps * 32u) return;
-    const uint32_t warps = min(min(kSpreadWarps, blockDim.x / 32u), uint32_t(perBlock));
+    if (!spread || perBlock > blockDim.x) return;
+    // As many warps of each block as it has work for: the blocks that start first
+    // would take all of it.
+    const bool few = perBlock <= kSpreadWarps * 32u;
+    const uint32_t warps = few ? min(min(kSpreadWarps, blockDim.x / 32u), uint32_t(perBlock))
+                               : (uint32_t(perBlock) + 31u) / 32u;
     exhausted = threadIdx.x / 32u >= warps;
+    if (!few) return;
     while (slice / 2u * warps >= perBlock && slice > 1u) slice /= 2u;
   }
 
